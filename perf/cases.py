@@ -3,7 +3,7 @@
 A case is a dict of plain values: what is called (``op``), the distribution of the sequence lengths, heads, head
 dimension, activation and options.  ``prepare`` makes the inputs of a case on the GPU from a seed (the lengths of a
 case are fixed by its ``len_seed``; the seed deals them out to the sequences and draws the values), ``run`` is one
-call through the public entry points of ``ads_model_kernel_library_b200.gdpa``.
+call through the public entry points of ``ads_model_kernel_library_b200.gdpa``; ``exact`` is the same in fp64.
 """
 import math
 
@@ -271,3 +271,85 @@ def tolerance(case):
     if case["op"] == "norms":
         return {"rel": 0.02, "max": 0.16}
     return {"rel": 0.01, "max": 0.1 if case["activation"] == "softmax" else 0.06}
+
+
+# ------------------------------------------------------------------------------------- the same pass in 64 bits
+
+
+def _mx_values(x, axis):
+    """What a block-scaled FP8 tensor of the values `x` ([rows, H, D], one sequence) stands for, in fp64: e4m3 elements, one
+    power of two per 32 of them along `axis`, the smallest with amax / scale <= 448."""
+    n = x.shape[axis]
+    pad = (-n) % 32
+    x = x.movedim(axis, -1).float()
+    g = torch.nn.functional.pad(x, (0, pad)).unflatten(-1, (-1, 32))
+    mantissa, exponent = torch.frexp(g.abs().amax(-1, keepdim=True) * (1.0 / 448.0))
+    scale = torch.exp2((exponent - (mantissa == 0.5).int()).double())
+    y = (g.double() / scale).float().to(torch.float8_e4m3fn).double() * scale
+    return y.flatten(-2)[..., :n].movedim(-1, axis)
+
+
+def _attention64(q, k, v, s):
+    """One sequence: [rows, H, D] tensors in fp64, K and V with a head for each query head."""
+    q, k, v = (t.transpose(0, 1) for t in (q, k, v))
+    x = q @ k.transpose(1, 2)
+    band = None
+    if s["window"] is not None:
+        i, j = torch.arange(x.shape[1], device=x.device).view(-1, 1), torch.arange(x.shape[2], device=x.device)
+        band = (i - j).abs() <= s["window"]
+    F = torch.nn.functional
+    if s["activation"] == "softmax":
+        p = torch.softmax(x * s["scale"], -1)
+    else:
+        if band is not None:
+            x = x * band
+        act = {"gelu_approx": lambda t: F.gelu(t, approximate="tanh"), "fast_gelu": lambda t: F.gelu(t, approximate="tanh"),
+               "silu": F.silu, "relu": F.relu}[s["activation"]]
+        p = act(x) * s["scale"]
+        if band is not None:
+            p = p * band
+    return (p @ v).transpose(0, 1)
+
+
+def exact(case, seed):
+    op, train = case["op"], case["train"]
+    s = prepare(dict(case, op="fp8") if op == "mxfp8" else case, seed)  # the inputs before they are quantised
+    H, Hk, D = case["heads"], case["kv_heads"], case["head_dim"]
+    qo, ko = s["qo"].tolist(), s["ko"].tolist()
+    lq, _ = _lengths(case)
+    owner = s["request_of"].tolist() if op == "shared_kv" else list(range(len(lq)))
+    out = torch.zeros(s["q"].shape, dtype=torch.float64, device="cuda")
+    names = [n for n in ("q", "k", "v") if s[n] is not None]
+    rows = {n: torch.zeros(s[n].shape, dtype=torch.float64, device="cuda") for n in names} if train else {}
+    vectors = {n: s[n].detach().double().requires_grad_(True) for n in ("ln_w", "ln_b", "rms_w")} if op == "norms" else {}
+    sums = {n: torch.zeros_like(t.detach()) for n, t in vectors.items()}
+    for b, kb in enumerate(owner):
+        at = {"q": slice(qo[b], qo[b + 1]), "k": slice(ko[kb], ko[kb + 1]), "v": slice(ko[kb], ko[kb + 1])}
+        if at["q"].start == at["q"].stop:
+            continue
+        x = {n: s[n].detach()[at[n]].double().requires_grad_(train) for n in names}
+        q, k = x["q"], x["k"]
+        k, v = (k, x["v"]) if "v" in x else k.split(D, -1)
+        if Hk != H:
+            k, v = (t.repeat_interleave(H // Hk, 1) for t in (k, v))
+        if op == "mxfp8":
+            q, k, v = _mx_values(s["q"][at["q"]], 2), _mx_values(s["k"][at["k"]], 2), _mx_values(s["v"][at["v"]], 0)
+        with torch.set_grad_enabled(train):
+            if op == "norms":
+                n = H * D
+                ln = torch.nn.functional.layer_norm(q.reshape(-1, n), (n,), vectors["ln_w"], vectors["ln_b"], 1e-5)
+                y = _attention64(ln.view(q.shape), k, v, s).reshape(-1, n) + ln
+                y = y * torch.rsqrt(y.square().mean(1, keepdim=True) + 1e-5) * vectors["rms_w"]
+                y = y.view(q.shape) + s["residual"][at["q"]].double()
+            else:
+                y = _attention64(q, k, v, s)
+        out[at["q"]] = y.detach()
+        if train:
+            wanted = [x[n] for n in names] + list(vectors.values())
+            got = torch.autograd.grad(y, wanted, s["dout"][at["q"]].double())
+            for n, g in zip(names + list(vectors), got):
+                if n in vectors:
+                    sums[n] += g
+                else:
+                    rows[n][at[n]] = g
+    return [out, *rows.values(), *sums.values()] if train else out
