@@ -1,0 +1,48 @@
+"""Edge sizes of the streaming kernels and of the schedule builder: remainders of their tiles, the smallest and largest
+sizes of each variant, values at the ends of the formats."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def G():
+    import ads_model_kernel_library_b200.gdpa as g
+
+    return g
+
+
+@pytest.mark.parametrize("rows,n", [(1, 8), (3, 256), (37, 512), (300, 520), (1001, 1024), (29, 1032), (150, 2048), (7, 4096), (33, 4104)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_norm_backward_at_the_edges_of_its_row_lengths(mode, rows, n):
+    """Rows of 8 ... 4104 values (one to eight warps a row, then the kernel for longer rows), against autograd in fp64.
+    dx is a bf16 tensor: half an ulp, 2^-9 of the value; the sums in fp32 add some 1e-6 of the largest term.  The column
+    sums are fp32 over `rows` terms."""
+    from ads_model_kernel_library_b200.gdpa.megakernel import NORM_EPS, norm_rows_backward
+
+    g = torch.Generator().manual_seed(rows + n)
+    x, dy, add = (torch.randn(rows, 1, n, generator=g).to(torch.bfloat16) for _ in range(3))
+    x = x + 0.5
+    w = 1 + 0.2 * torch.randn(n, generator=g)
+    want_dw = n <= 4096
+    xd, wd, bd = x.double().view(rows, n).requires_grad_(True), w.double().requires_grad_(True), torch.zeros(n).double().requires_grad_(True)
+    mean = xd.mean(1, keepdim=True)
+    if mode == 0:
+        rstd = torch.rsqrt(xd.square().mean(1, keepdim=True) + NORM_EPS)
+        y = xd * rstd * wd
+    else:
+        rstd = torch.rsqrt((xd - mean).square().mean(1, keepdim=True) + NORM_EPS)
+        y = (xd - mean) * rstd * wd + bd
+    y.backward((dy.double() + (add.double() if mode == 1 else 0)).view(rows, n))
+    dx, dw, db = norm_rows_backward(mode, dy.cuda(), add.cuda() if mode == 1 else None, x.cuda(), w.cuda(),
+                                    mean.detach().float().view(-1).cuda(), rstd.detach().float().view(-1).cuda(),
+                                    want_dweight=want_dw, want_dbias=want_dw and mode == 1)
+    torch.cuda.synchronize()
+    ref = xd.grad.view_as(dx)
+    assert ((dx.cpu().double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all()
+    if want_dw:
+        tol = 1e-6 * rows ** 0.5 * 16 + 1e-5  # fp32 sums of terms of a few units
+        assert ((dw.cpu().double() - wd.grad).abs() <= tol * (1 + wd.grad.abs())).all()
+        if mode == 1:
+            assert ((db.cpu().double() - bd.grad).abs() <= tol * (1 + bd.grad.abs())).all()
