@@ -40,52 +40,81 @@ __device__ __forceinline__ void seq_geometry(const SchedArgs& a, int b, int& nbl
   if (weight > kBins - 1) weight = kBins - 1;
 }
 
+// Latency-bound: one block, a few thousand items, and the forward or backward kernel waits for it.  What it costs is the
+// chain of dependent steps, so: only the bins that a sequence of the given maximum length can have are cleared and
+// scanned (17 of 4096 for 2048 tokens), the scan gives each thread its own run of neighbouring bins (a warp reads
+// consecutive words, no bank conflicts) instead of one warp walking all of them, and the items of a chunk of 1024
+// sequences are written by all warps together, 32 consecutive items (512 bytes) per store, instead of each thread
+// writing the items of one sequence one after another (13 us for 8 sequences, 26 us for 1024, a call of 256 short
+// sequences 86.7 -> 81.8 us in all).
 __global__ void __launch_bounds__(kSchedThreads, 1) gdpa_build_schedule_kernel(const SchedArgs a) {
   __shared__ int hist[kBins];
-  __shared__ int total;
-  for (int i = threadIdx.x; i < kBins; i += kSchedThreads) hist[i] = 0;
+  __shared__ int warp_sum[kSchedThreads / 32];
+  __shared__ int4 seq[kSchedThreads];  // of the sequences of one chunk: first slot, blocks, weight, -
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int longest = a.mode == 0 ? a.max_kv : a.max_q;
+  const int bins = min(kBins, (longest > 0 ? (longest - 1) / kTile + 1 : 0) + 1);  // weights 0 .. bins - 1
+  const long long cap = a.capacity_items;
+  for (int i = t; i < bins; i += kSchedThreads) hist[i] = 0;
   __syncthreads();
-  for (int b = threadIdx.x; b < a.batch; b += kSchedThreads) {
-    int nblk, w;
+  int nblk = 0, w = 0;  // of this thread's sequence of the last chunk: the only one unless the batch is large
+  for (int b = t; b < a.batch; b += kSchedThreads) {
     seq_geometry(a, b, nblk, w);
     if (nblk > 0) atomicAdd(&hist[w], nblk * a.heads);
   }
   __syncthreads();
-  // Exclusive prefix over bins from the heaviest down: hist[w] becomes the first slot of weight w.
-  if (threadIdx.x < 32) {
-    // Each lane owns a contiguous run of bins (heaviest first); lane totals are scanned by shuffles.
-    constexpr int per = kBins / 32;
-    const int hi = kBins - 1 - threadIdx.x * per;  // this lane walks hi, hi-1, ..., hi-per+1
-    int sum = 0;
-    for (int i = 0; i < per; ++i) sum += hist[hi - i];
-    int incl = sum;
-    for (int d = 1; d < 32; d <<= 1) {
-      int n = __shfl_up_sync(0xffffffffu, incl, d);
-      if (threadIdx.x >= d) incl += n;
-    }
-    int run = incl - sum;
-    for (int i = 0; i < per; ++i) {
-      const int c = hist[hi - i];
-      hist[hi - i] = run;
-      run += c;
-    }
-    if (threadIdx.x == 31) total = incl;
+  // Exclusive prefix over bins from the heaviest down: hist[w] becomes the first slot of weight w.  Thread t owns the
+  // `per` bins from bins - 1 - t * per down.
+  const int per = (bins + kSchedThreads - 1) / kSchedThreads;
+  const int hi = bins - 1 - t * per;
+  int sum = 0;
+  for (int i = 0; i < per; ++i) sum += hi - i >= 0 ? hist[hi - i] : 0;
+  int incl = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int n = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += n;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  // every warp scans the 32 warp totals for itself
+  int before = warp_sum[lane];
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int n = __shfl_up_sync(0xffffffffu, before, d);
+    if (lane >= d) before += n;
+  }
+  const int total = __shfl_sync(0xffffffffu, before, 31);
+  before = __shfl_sync(0xffffffffu, before, warp > 0 ? warp - 1 : 0);
+  int run = incl - sum + (warp > 0 ? before : 0);
+  for (int i = 0; i < per; ++i) {
+    if (hi - i < 0) break;
+    const int c = hist[hi - i];
+    hist[hi - i] = run;
+    run += c;
   }
   __syncthreads();
-  const long long cap = a.capacity_items;
   int4* items = reinterpret_cast<int4*>(a.sched + kSchedHeaderInts);
-  for (int b = threadIdx.x; b < a.batch; b += kSchedThreads) {
-    int nblk, w;
-    seq_geometry(a, b, nblk, w);
-    if (nblk == 0) continue;
-    const int base = atomicAdd(&hist[w], nblk * a.heads);
-    for (int h = 0; h < a.heads; ++h)
-      for (int blk = 0; blk < nblk; ++blk) {
-        const long long slot = static_cast<long long>(base) + h * nblk + blk;
-        if (slot < cap) items[slot] = make_int4(b, h, blk, w);
+  for (int b0 = 0; b0 < a.batch; b0 += kSchedThreads) {
+    const int n = min(kSchedThreads, a.batch - b0);
+    if (t < n) {
+      if (a.batch > kSchedThreads) seq_geometry(a, b0 + t, nblk, w);
+      const int count = nblk * a.heads;
+      seq[t] = make_int4(count > 0 ? atomicAdd(&hist[w], count) : 0, nblk, w, 0);
+    }
+    __syncthreads();
+    for (int i = warp; i < n; i += kSchedThreads / 32) {
+      const int4 sq = seq[i];
+      const int count = sq.y * a.heads;
+      for (int k = lane; k < count; k += 32) {
+        const long long slot = static_cast<long long>(sq.x) + k;
+        const int h = k / sq.y;
+        if (slot < cap) items[slot] = make_int4(b0 + i, h, k - h * sq.y, sq.z);
       }
+    }
+    __syncthreads();
   }
-  if (threadIdx.x == 0) {
+  if (t == 0) {
     a.sched[0] = static_cast<int>(total < cap ? total : cap);
     a.sched[1] = a.mode;
     a.sched[2] = total;  // items the batch needs; larger than [0] only if the buffer was too small

@@ -1,5 +1,6 @@
 """Edge sizes of the streaming kernels and of the schedule builder: remainders of their tiles, the smallest and largest
 sizes of each variant, values at the ends of the formats."""
+import numpy as np
 import pytest
 import torch
 
@@ -46,3 +47,30 @@ def test_norm_backward_at_the_edges_of_its_row_lengths(mode, rows, n):
         assert ((dw.cpu().double() - wd.grad).abs() <= tol * (1 + wd.grad.abs())).all()
         if mode == 1:
             assert ((db.cpu().double() - bd.grad).abs() <= tol * (1 + bd.grad.abs())).all()
+
+
+def _schedule(qo, ko, mode, heads, max_q, max_kv, kv_index=None):
+    from ads_model_kernel_library_b200.gdpa import ops
+
+    total = int((qo if mode != 1 else ko)[-1])
+    s = ops._build_schedule(mode, qo, ko, qo.numel() - 1, heads, total, max_q, max_kv, kv_index).cpu()
+    return s[:4].tolist(), s[4:4 + 4 * int(s[0])].view(-1, 4)
+
+
+@pytest.mark.parametrize("batch", [1, 31, 1023, 1024, 1025, 2500])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_schedule_lists_every_block_once_longest_first(mode, batch):
+    rng = np.random.default_rng(batch)
+    lq, lk = rng.integers(0, 700, batch), rng.integers(0, 3000, batch)
+    lq[0] = lk[0] = 700
+    qo, ko = (torch.tensor(np.concatenate([[0], np.cumsum(n)])).cuda() for n in (lq, lk))
+    heads, max_q, max_kv = 3, 600, 2500
+    header, items = _schedule(qo, ko, mode, heads, max_q, max_kv)
+    tiles = lambda n, t: -(-n // t)  # noqa: E731
+    cq, ck = np.minimum(lq, max_q), np.minimum(lk, max_kv)
+    blocks, weight = (tiles(cq, 256), tiles(ck, 128)) if mode == 0 else (tiles(ck, 128), tiles(cq, 128))
+    want = [(b, h, k, weight[b]) for b in range(batch) for h in range(heads) for k in range(blocks[b])]
+    assert header[0] == header[2] == len(want) and header[1] == mode and header[3] == 0
+    assert sorted(map(tuple, items.tolist())) == want
+    w = items[:, 3]
+    assert bool((w[1:] <= w[:-1]).all())
