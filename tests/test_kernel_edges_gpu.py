@@ -4,6 +4,8 @@ import numpy as np
 import pytest
 import torch
 
+from tests._util import assert_close
+
 pytestmark = pytest.mark.gpu
 
 
@@ -74,3 +76,27 @@ def test_schedule_lists_every_block_once_longest_first(mode, batch):
     assert sorted(map(tuple, items.tolist())) == want
     w = items[:, 3]
     assert bool((w[1:] <= w[:-1]).all())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("tokens", [1, 63, 64, 129, 1000])
+@pytest.mark.parametrize("shift", [0, 2])
+def test_softmax_backward_for_any_number_of_tokens_and_alignment_of_the_output(D, tokens, shift):
+    """rowsum(dO * O) is taken over blocks of 64 / 128 tokens, by 16-byte words where the output is aligned to them: dQ of
+    the whole backward against autograd of the fp64 attention, within the bf16 bound of the kernels (2e-2)."""
+    import math
+
+    g = torch.Generator().manual_seed(tokens + D)
+    H, kv = 3, 77
+    q, do = (torch.randn(tokens, H, D, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    k, v = (torch.randn(kv, H, D, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    qo, ko = torch.tensor([0, tokens]).cuda(), torch.tensor([0, kv]).cuda()
+    scale = 1 / math.sqrt(D)
+    o, lse = torch.ops.gdpa.generalized_dot_product_attention_softmax(q, k, v, qo, ko, tokens, kv, scale)
+    moved = torch.empty(o.numel() + shift, dtype=o.dtype, device="cuda")[shift:].view(o.shape).copy_(o)
+    dq = torch.ops.gdpa.generalized_dot_product_attention_backward(do, q, k, v, qo, ko, tokens, kv, scale, 100, moved, lse)[0]
+    torch.cuda.synchronize()
+    q64 = q.double().requires_grad_(True)
+    p = torch.softmax(torch.einsum("qhd,khd->hqk", q64, k.double()) * scale, -1)
+    torch.einsum("hqk,khd->qhd", p, v.double()).backward(do.double())
+    assert_close(dq, q64.grad, "dQ")
