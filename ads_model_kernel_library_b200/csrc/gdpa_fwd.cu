@@ -49,9 +49,9 @@ enum FwdBar : int {
   B_KV_FULL = 4,                       // [kKvStages]
   B_KV_EMPTY = 4 + kKvStages,          // [kKvStages]
   B_S_FULL = 4 + 2 * kKvStages,        // [2] MMA commit -> activation group
-  B_P_FULL = 6 + 2 * kKvStages,        // [2] activation group (128 arrivals) -> MMA
+  B_P_FULL = 6 + 2 * kKvStages,        // [2] activation group (256 arrivals) -> MMA
   B_O_FULL = 8 + 2 * kKvStages,        // [2] MMA commit -> epilogue
-  B_O_EMPTY = 10 + 2 * kKvStages,      // [2] epilogue (128 arrivals) -> MMA
+  B_O_EMPTY = 10 + 2 * kKvStages,      // [2] epilogue (256 arrivals) -> MMA
   B_L_FULL = 12 + 2 * kKvStages,       // [2] softmax: activation group -> epilogue (row sums)
   B_M_FULL = 14 + 2 * kKvStages,       // [2] softmax, wide layout: both column halves have published their row maxima
   B_LD_TMP = 16 + 2 * kKvStages,       // the loader's own: a ragged tile has landed and can have its padding rows zeroed
@@ -142,13 +142,9 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < B_COUNT; ++i) {
-      const bool many = (i >= B_P_FULL && i < B_P_FULL + 2) || (i >= B_O_EMPTY && i < B_O_EMPTY + 2) ||
-                        (i >= B_L_FULL && i < B_L_FULL + 2);
-      uint32_t cnt = many ? 128u : 1u;
-      if ((i >= B_P_FULL && i < B_P_FULL + 2) || (i >= B_O_EMPTY && i < B_O_EMPTY + 2) ||
-          (i >= B_L_FULL && i < B_L_FULL + 2) || (i >= B_M_FULL && i < B_M_FULL + 2))
-        cnt = kStageThreads;
-      mbar_init(bar_base + 8u * i, cnt);
+      const bool by_threads = (i >= B_P_FULL && i < B_P_FULL + 2) || (i >= B_O_EMPTY && i < B_O_EMPTY + 2) ||
+                            (i >= B_L_FULL && i < B_L_FULL + 2) || (i >= B_M_FULL && i < B_M_FULL + 2);
+      mbar_init(bar_base + 8u * i, by_threads ? kStageThreads : 1u);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -400,7 +396,6 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         // bias = log2(V-block scale), so P contains the V scale and uses the whole e4m3 range; the row
         // sum divides it out again.
         constexpr float kThr = FP8 ? 1.f : 8.f;
-        constexpr float kPScale = FP8 ? 128.f : 1.f;
         constexpr float kLog2e = 1.4426950408889634f;
         float* rowmax = reinterpret_cast<float*>(smem + L::kRowMaxOff);
         float* rowsum = reinterpret_cast<float*>(smem + L::kRowSumOff);
@@ -442,9 +437,17 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
             if (ch == 0) tmem_ld32(s_tmem + 32, rb);
             // a chunk wholly inside [clo, chi) for every row of the warp needs no predicates; without a band
             // the lower bound is 0
-            if (__all_sync(0xffffffffu, clo <= ch * 32 && chi >= (ch + 1) * 32)) {
+            // (scale >= 0: the largest c * S is c times the largest S, one three-way maximum per two columns; with the
+            // packed arithmetic of pass 2 about 190 instead of 350 issue slots per warp and tile: FP8 forward 5.11 -> 4.96 ms,
+            // bf16 training step 1.96 -> 1.94 ms)
+            if (a.scale >= 0.f && __all_sync(0xffffffffu, clo <= ch * 32 && chi >= (ch + 1) * 32)) {
+              float m0 = __uint_as_float(cur[0]), m1 = __uint_as_float(cur[1]);
 #pragma unroll
-              for (int i = 0; i < 32; ++i) pmax = fmaxf(pmax, __uint_as_float(cur[i]) * c);
+              for (int i = 2; i < 32; i += 4) {
+                m0 = max3(m0, __uint_as_float(cur[i]), __uint_as_float(cur[i + 1]));
+                if (i + 2 < 32) m1 = max3(m1, __uint_as_float(cur[i + 2]), __uint_as_float(cur[i + 3]));
+              }
+              pmax = fmaxf(pmax, fmaxf(m0, m1) * c);
             } else if (a.window < 0) {
 #pragma unroll
               for (int i = 0; i < 32; ++i) {
@@ -486,8 +489,10 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
           }
           // pass 2: reload the scores, P = exp2(c S + bias - m), partial row sum, quantise, store over
           // columns of this half that have been read
-          const float off = (m_used == -INFINITY) ? 0.f : bias - m_used;  // a row may have seen no column yet
-          float psum = 0.f;
+          // (FP8: P is stored times 2^7, which goes into the exponent)
+          const float off = (m_used == -INFINITY) ? 0.f : bias - m_used + (FP8 ? 7.f : 0.f);  // a row may have seen no column yet
+          const uint64_t c2 = pack_f32x2(c, c), off2 = pack_f32x2(off, off);
+          uint64_t psum2 = 0;  // partial row sums of the even and the odd columns
           tmem_ld32(s_tmem, ra);
 #pragma unroll
           for (int ch = 0; ch < 2; ++ch) {
@@ -498,25 +503,31 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
             // P of this chunk with the column test `inside`; three instantiations so that the common case (the
             // chunk wholly inside [clo, chi) for every row of the warp) carries no predicates at all
             auto emit = [&](auto inside) {
-              auto prob = [&](int i) {
-                const float e = ex2_approx(fmaf(__uint_as_float(cur[i]), c, off));
-                const float p = inside(i) ? e : 0.f;
-                psum += p;
-                return p;
+              auto prob2 = [&](int i, float& p0, float& p1) {  // columns 2i and 2i + 1 of the chunk
+                float e0, e1;
+                unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(cur[2 * i]), __uint_as_float(cur[2 * i + 1])), c2, off2), e0, e1);
+                e0 = ex2_approx(e0);
+                e1 = ex2_approx(e1);
+                p0 = inside(2 * i) ? e0 : 0.f;
+                p1 = inside(2 * i + 1) ? e1 : 0.f;
+                psum2 = add_f32x2(psum2, pack_f32x2(p0, p1));
               };
               if constexpr (FP8) {
                 uint32_t pk[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                  const float p0 = prob(4 * i), p1 = prob(4 * i + 1), p2 = prob(4 * i + 2), p3 = prob(4 * i + 3);
-                  pk[i] = pack_e4m3x4(p0 * kPScale, p1 * kPScale, p2 * kPScale, p3 * kPScale);
+                  float p0, p1, p2, p3;
+                  prob2(2 * i, p0, p1);
+                  prob2(2 * i + 1, p2, p3);
+                  pk[i] = pack_e4m3x4(p0, p1, p2, p3);
                 }
                 tmem_st8(s_tmem + ch * 8, pk);
               } else {
                 uint32_t pk[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                  const float p0 = prob(2 * i), p1 = prob(2 * i + 1);
+                  float p0, p1;
+                  prob2(i, p0, p1);
                   pk[i] = pack_bf16x2(p0, p1);
                 }
                 tmem_st16(s_tmem + ch * 16, pk);
@@ -526,16 +537,18 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
             else if (a.window < 0) emit([&](int i) { return ch * 32 + i < chi; });  // without a band the lower bound is 0
             else emit([&](int i) { return ch * 32 + i >= clo && ch * 32 + i < chi; });
           }
-          row_sum = fmaf(psum, inv_sv, row_sum);
+          float psum_even, psum_odd;
+          unpack_f32x2(psum2, psum_even, psum_odd);
+          row_sum = fmaf(psum_even + psum_odd, inv_sv, row_sum);
           tmem_wait_st();
           tc_fence_before();
           mbar_arrive(bar_base + 8u * (B_P_FULL + s));
         }
         // both halves publish their partial row sums; each then divides its half of O by the total
-        rowsum[(s * 2 + half) * kTile + row] = row_sum * kPScale;
+        rowsum[(s * 2 + half) * kTile + row] = row_sum;
         mbar_arrive(bar_base + 8u * (B_L_FULL + s));
         GDPA_WAIT_WARP(B_L_FULL + s, o_phase, ST_ROLE_EPI);
-        const float l_total = row_sum * kPScale + reinterpret_cast<volatile float*>(rowsum)[(s * 2 + (half ^ 1)) * kTile + row];
+        const float l_total = row_sum + reinterpret_cast<volatile float*>(rowsum)[(s * 2 + (half ^ 1)) * kTile + row];
         inv_l = l_total > 0.f ? 1.f / l_total : 0.f;  // a row whose band holds no key gives zeros
         if constexpr (!FP8) {
           // log-sum-exp of the scaled scores in base 2, for the softmax backward (+inf for a row without

@@ -100,3 +100,26 @@ def test_softmax_backward_for_any_number_of_tokens_and_alignment_of_the_output(D
     p = torch.softmax(torch.einsum("qhd,khd->hqk", q64, k.double()) * scale, -1)
     torch.einsum("hqk,khd->qhd", p, v.double()).backward(do.double())
     assert_close(dq, q64.grad, "dQ")
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("scale", [-0.1, 0.0, 0.1])
+def test_softmax_forward_for_every_sign_of_the_scale(D, scale):
+    """The row maximum of c * S is c times the maximum of S only for c >= 0; KV lengths at the edges of the 32- and
+    64-column chunks.  Against the fp64 softmax within the bf16 bound of the kernels."""
+    import ads_model_kernel_library_b200.gdpa as G
+
+    g = torch.Generator().manual_seed(D)
+    lk = [1, 31, 32, 33, 64, 65, 127, 128, 129, 400]
+    lq = [1, 40, 128, 129, 300, 7, 256, 64, 200, 130]
+    qo, ko = (torch.tensor(np.concatenate([[0], np.cumsum(n)])) for n in (lq, lk))
+    q = (torch.randn(int(qo[-1]), 2, D, generator=g) * 2).to(torch.bfloat16)
+    k, v = ((torch.randn(int(ko[-1]), 2, D, generator=g) * 2).to(torch.bfloat16) for _ in range(2))
+    o = G.generalized_dot_product_attention(q.cuda(), k.cuda(), v.cuda(), qo.cuda(), ko.cuda(), max(lq), max(lk), qk_scale=scale,
+                                            activation="softmax")
+    torch.cuda.synchronize()
+    assert G.kernel_status() == 0
+    for b in range(len(lq)):
+        qb, (kb, vb) = q[qo[b]:qo[b + 1]].double(), (t[ko[b]:ko[b + 1]].double() for t in (k, v))
+        p = torch.softmax(torch.einsum("qhd,khd->hqk", qb, kb) * scale, -1)
+        assert_close(o[qo[b]:qo[b + 1]], torch.einsum("hqk,khd->qhd", p, vb), f"O[{lq[b]}, {lk[b]}]")
