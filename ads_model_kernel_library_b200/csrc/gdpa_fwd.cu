@@ -41,6 +41,7 @@ namespace {
 // activation warps per SM sub-partition and Q tile halve the activation time.
 constexpr int kFwdThreads = 20 * 32;
 constexpr int kKvStages = 4;
+constexpr int kWorkSlots = 4;
 
 // Barrier indices inside the shared barrier array.
 enum FwdBar : int {
@@ -55,7 +56,9 @@ enum FwdBar : int {
   B_L_FULL = 12 + 2 * kKvStages,       // [2] softmax: activation group -> epilogue (row sums)
   B_M_FULL = 14 + 2 * kKvStages,       // [2] softmax, wide layout: both column halves have published their row maxima
   B_LD_TMP = 16 + 2 * kKvStages,       // the loader's own: a ragged tile has landed and can have its padding rows zeroed
-  B_COUNT = 17 + 2 * kKvStages
+  B_WORK_FULL = 17 + 2 * kKvStages,               // [kWorkSlots] the loader has published a work item
+  B_WORK_EMPTY = 17 + 2 * kKvStages + kWorkSlots, // [kWorkSlots] the MMA thread and the 16 activation warps have read it
+  B_COUNT = 17 + 2 * kKvStages + 2 * kWorkSlots
 };
 
 template <int D, int EB>
@@ -82,7 +85,8 @@ struct FwdSmem {
   static_assert(kStatBytes + 16 * kNarrowSlabBytes <= 16 * kOutSlabBytes, "the narrow slabs fit in the staging region");
   static constexpr int kBarOff = kOutOff + 16 * kOutSlabBytes;
   static_assert(16 * kOutSlabBytes >= kStatBytes, "the softmax arrays fit in the staging region");
-  static constexpr int kTmemPtrOff = kBarOff + B_COUNT * 8;
+  static constexpr int kWorkOff = (kBarOff + B_COUNT * 8 + 15) / 16 * 16;  // WorkSlot[kWorkSlots]: the work items in flight
+  static constexpr int kTmemPtrOff = kWorkOff + kWorkSlots * 48;
   static constexpr int kAbortOff = kTmemPtrOff + 4;
   static constexpr int kBytes = kAbortOff + 4;
   static constexpr int kDynBytes = kBytes + 1024;        // slack to align the base to 1024 bytes
@@ -144,7 +148,8 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
     for (int i = 0; i < B_COUNT; ++i) {
       const bool by_threads = (i >= B_P_FULL && i < B_P_FULL + 2) || (i >= B_O_EMPTY && i < B_O_EMPTY + 2) ||
                             (i >= B_L_FULL && i < B_L_FULL + 2) || (i >= B_M_FULL && i < B_M_FULL + 2);
-      mbar_init(bar_base + 8u * i, by_threads ? kStageThreads : 1u);
+      const bool by_readers = i >= B_WORK_EMPTY && i < B_WORK_EMPTY + kWorkSlots;
+      mbar_init(bar_base + 8u * i, by_threads ? kStageThreads : by_readers ? 1u + kActWarps : 1u);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -164,6 +169,34 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
   const uint32_t tmem_base = *tmem_ptr;
   const int n_items = a.sched[0];
   const SeqLimits lim = {a.total_q, a.total_kv, a.kv_batch};
+
+  // The loader warp walks the list, reads an item and its sequence's offsets (two dependent trips to memory, with FP8
+  // a third for the rows of the block scales) and publishes what they say through a small ring in shared memory, an item
+  // ahead of its use; the MMA thread and the activation warps start on an item with two or three shared-memory loads
+  // instead of making those trips each.  FP8 forward 4.96 -> 4.83 ms, the norm pipeline's step 7.77 -> 7.71 ms, the plain
+  // forward of long and short items unchanged.
+  // Slot: {head, Q block, first Q row, first KV row}, {lq, lkv, first KV tile, KV tiles}, {Q scale row of Q tile 0, KV
+  // scale row of KV tile 0 (FP8), -, -}; head -1 ends the walk.
+  int4* const work_ring = reinterpret_cast<int4*>(smem + L::kWorkOff);
+  uint32_t work_pos = 0;  // items this role has taken: ring slot = work_pos % kWorkSlots, parity = (work_pos / kWorkSlots) & 1
+  struct Item {
+    int h, blk, q_start, kv_start, lq, lkv, j0, nkv, q_scale0, kv_scale0;
+  };
+  // Consumer side: this role's next work item; h = -1 at the end of the list, -2 if the wait ran out.
+  // `warp_wide`: called by a whole warp, whose lane 0 releases the slot.
+  auto take_work_item = [&](int role, bool warp_wide) -> Item {
+    const uint32_t slot = work_pos % kWorkSlots, parity = (work_pos / kWorkSlots) & 1u;
+    ++work_pos;
+    bool ok = mbar_wait(bar_base + 8u * (B_WORK_FULL + slot), parity, abort_flag, a.status, ((B_WORK_FULL + slot) << 8) | role);
+    if (warp_wide) ok = __all_sync(0xffffffffu, ok);
+    if (!ok) return Item{-2, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    const int4 u = work_ring[3 * slot], v = work_ring[3 * slot + 1];
+    int4 x = make_int4(0, 0, 0, 0);
+    if (FP8) x = work_ring[3 * slot + 2];
+    if (warp_wide) __syncwarp();
+    if (!warp_wide || lane == 0) mbar_arrive(bar_base + 8u * (B_WORK_EMPTY + slot));
+    return Item{u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w, x.x, x.y};
+  };
 
   // Operand format code: 1 = bf16 for kind::f16, 0 = e4m3 for kind::f8f6f4.
   constexpr uint32_t kFmt = FP8 ? 0u : 1u;
@@ -207,16 +240,44 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         return true;
       };
       WorkWalker walker(n_items);
-      int idx;
-      while (walker.next(idx)) {
-        const Work w = load_work(a.sched, idx, a.q_off, a.kv_off, a.off64, a.max_q, a.max_kv, lim, a.kv_index);
-        int j0, nkv;  // first KV tile and number of KV tiles this item visits
-        fwd_kv_range(w, a.window, j0, nkv);
+      // producer side of the work ring: the slot must have been read by every consumer of its previous use
+      auto next_item = [&](Item& it) -> bool {
+        const uint32_t slot = work_pos % kWorkSlots, parity = (work_pos / kWorkSlots) & 1u;
+        it = Item{-1, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+        int i;
+        if (walker.next(i)) {
+          const Work w = load_work(a.sched, i, a.q_off, a.kv_off, a.off64, a.max_q, a.max_kv, lim, a.kv_index);
+          it.h = w.h, it.blk = w.blk;
+          it.q_start = static_cast<int>(w.q_start), it.kv_start = static_cast<int>(w.kv_start);
+          it.lq = w.lq, it.lkv = w.lkv;
+          fwd_kv_range(w, a.window, it.j0, it.nkv);
+          if constexpr (FP8) {
+            it.q_scale0 = static_cast<int>(load_offset(a.q_blk_off, w.b, a.off64)) + w.blk * 2;
+            it.kv_scale0 = static_cast<int>(load_offset(a.kv_blk_off, w.kb, a.off64));
+          }
+        }
+        const bool ok = mbar_wait(bar_base + 8u * (B_WORK_EMPTY + slot), parity ^ 1u, abort_flag, a.status,
+                                  ((B_WORK_EMPTY + slot) << 8) | ST_ROLE_LOAD);
+        if (!__all_sync(0xffffffffu, ok)) return false;
+        if (lane == 0) {
+          work_ring[3 * slot] = make_int4(it.h, it.blk, it.q_start, it.kv_start);
+          work_ring[3 * slot + 1] = make_int4(it.lq, it.lkv, it.j0, it.nkv);
+          if (FP8) work_ring[3 * slot + 2] = make_int4(it.q_scale0, it.kv_scale0, 0, 0);
+          mbar_arrive(bar_base + 8u * (B_WORK_FULL + slot));
+        }
+        ++work_pos;
+        return true;
+      };
+      Item w, w_next;
+      if (!next_item(w)) goto role_done;
+      for (; w.h >= 0; w = w_next) {
+        if (!next_item(w_next)) goto role_done;
+        const int j0 = w.j0, nkv = w.nkv;  // first KV tile and number of KV tiles this item visits
         if (nkv == 0) continue;
         const int q0 = w.blk * kFwdQBlock;
         const int nst = (w.lq - q0 > kTile) ? 2 : 1;
-        const int q_row = static_cast<int>(w.q_start) + q0;
-        const int kv_row = static_cast<int>(w.kv_start) + j0 * kTile;
+        const int q_row = w.q_start + q0;
+        const int kv_row = w.kv_start + j0 * kTile;
         // Issue order Q0, K0, Q1, V0, K1, V1, ...
         for (int step = 0; step < 2 * nkv + 2; ++step) {
           if (step == 0 || step == 2) {
@@ -282,12 +343,13 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
           else umma_ts_f16(d_tmem, a_tmem + a_col, umma_desc_advance(db, kk * kRowsPerSlice * 128), kIdescPV, acc);
         }
       };
-      WorkWalker walker(n_items);
-      int idx;
-      while (walker.next(idx)) {
-        const Work w = load_work(a.sched, idx, a.q_off, a.kv_off, a.off64, a.max_q, a.max_kv, lim, a.kv_index);
-        int j0, nkv;
-        fwd_kv_range(w, a.window, j0, nkv);
+      while (true) {
+        const Item w = take_work_item(ST_ROLE_MMA, false);
+        if (w.h < 0) {
+          if (w.h == -2) goto role_done;
+          break;
+        }
+        const int nkv = w.nkv;
         if (nkv == 0) continue;
         const int nst = (w.lq - w.blk * kFwdQBlock > kTile) ? 2 : 1;
         // First S tiles: S_s = Q_s K_0^T.
@@ -354,18 +416,19 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
     const float scale = a.scale, hscale = 0.5f * a.scale;
     uint32_t s_phase = 0, o_phase = 0;
     int tr = 0;
-    WorkWalker walker(n_items);
-    int idx;
-    while (walker.next(idx)) {
-      const Work w = load_work(a.sched, idx, a.q_off, a.kv_off, a.off64, a.max_q, a.max_kv, lim, a.kv_index);
-      int j0, nkv;
-      fwd_kv_range(w, a.window, j0, nkv);
+    while (true) {
+      const Item w = take_work_item(ST_ROLE_ACT, true);
+      if (w.h < 0) {
+        if (w.h == -2) goto role_done;
+        break;
+      }
+      const int j0 = w.j0, nkv = w.nkv;
       const int q0 = w.blk * kFwdQBlock;
       const int nst = (w.lq - q0 > kTile) ? 2 : 1;
       if (s >= nst) continue;
       const int qr = q0 + s * kTile + row;
       const bool row_valid = qr < w.lq;
-      const long long o_elem = ((w.q_start + qr) * a.heads + w.h) * static_cast<long long>(D) + half * (D / 2);
+      const long long o_elem = (static_cast<long long>(w.q_start + qr) * a.heads + w.h) * D + half * (D / 2);
       uint4* dst = reinterpret_cast<uint4*>(a.o + o_elem);
       // fused epilogue of the norm pipeline: x = O + residual, and the sum of x^2 over this thread's half row is
       // added to the row's entry of row_sumsq (the RMS norm over all heads is finished by a second kernel)
@@ -403,8 +466,8 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         float sq = 1.f;
         long long kv_blk0 = 0;
         if constexpr (FP8) {
-          sq = a.q_scales[(load_offset(a.q_blk_off, w.b, a.off64) + w.blk * 2 + s) * a.heads + w.h];
-          kv_blk0 = load_offset(a.kv_blk_off, w.kb, a.off64);
+          sq = a.q_scales[static_cast<long long>(w.q_scale0 + s) * a.heads + w.h];
+          kv_blk0 = w.kv_scale0;
         }
         for (int j = 0; j < nkv; ++j) {
           // columns [clo, chi) of this warp's 64 take part: inside the KV length and inside the band
@@ -564,8 +627,8 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
       long long fp8_kv_blk0 = 0;
       if constexpr (FP8 && !kSoftmax) {
         const int hkv = w.h / a.kv_group;
-        fp8_sq = a.q_scales[(load_offset(a.q_blk_off, w.b, a.off64) + w.blk * 2 + s) * a.heads + w.h];
-        fp8_kv_blk0 = load_offset(a.kv_blk_off, w.kb, a.off64);
+        fp8_sq = a.q_scales[static_cast<long long>(w.q_scale0 + s) * a.heads + w.h];
+        fp8_kv_blk0 = w.kv_scale0;
         float sv_max = 0.f;
         for (int j = 0; j < nkv; ++j) sv_max = fmaxf(sv_max, a.v_scales[(fp8_kv_blk0 + j0 + j) * a.kv_heads + hkv]);
         fp8_inv_svmax = sv_max > 0.f ? 1.f / sv_max : 0.f;
@@ -653,7 +716,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
             for (int i = 0; i < 4; ++i) {
               const int p = i * 32 + lane;
               rres[c][i] = *reinterpret_cast<const uint4*>(
-                  a.residual + ((w.q_start + (qr - lane) + (p >> 2)) * a.heads + w.h) * static_cast<long long>(D) + half * (D / 2) +
+                  a.residual + (static_cast<long long>(w.q_start + (qr - lane) + (p >> 2)) * a.heads + w.h) * D + half * (D / 2) +
                   c * 32 + (p & 3) * 8);
             }
         }
@@ -695,7 +758,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            tma_store_3d(&tm_o.m, slab, half * (D / 2) + c * 32, w.h, static_cast<int>(w.q_start) + qr);
+            tma_store_3d(&tm_o.m, slab, half * (D / 2) + c * 32, w.h, w.q_start + qr);
             tma_store_commit();
           }
         } else if (kNarrowOut && slab_rows >= 32) {
@@ -720,7 +783,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              tma_store_3d(&tm_o.m, slab, half * (D / 2) + c * 32 + h2 * 16, w.h, static_cast<int>(w.q_start) + qr);
+              tma_store_3d(&tm_o.m, slab, half * (D / 2) + c * 32 + h2 * 16, w.h, w.q_start + qr);
               tma_store_commit();
             }
           }
@@ -760,7 +823,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            tma_store_3d(&tm_o.m, slab, half * (D / 2) + c * 32, w.h, static_cast<int>(w.q_start) + qr);
+            tma_store_3d(&tm_o.m, slab, half * (D / 2) + c * 32, w.h, w.q_start + qr);
             tma_store_commit();
           }
         } else if (row_valid) {
