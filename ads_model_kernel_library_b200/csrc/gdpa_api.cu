@@ -178,7 +178,8 @@ size_t gdpa_bwd_workspace_bytes(int64_t total_q, int32_t heads, int32_t head_dim
 int gdpa_build_schedule(const GdpaSchedParams* p, gdpa_stream_t stream) {
   if (p == nullptr || p->struct_size != sizeof(GdpaSchedParams)) return GDPA_ERR_BAD_ARG;
   if (p->batch < 0 || p->heads <= 0 || p->schedule == nullptr) return GDPA_ERR_BAD_ARG;
-  if (p->mode != GDPA_SCHED_FWD && p->mode != GDPA_SCHED_BWD) return GDPA_ERR_BAD_ARG;
+  if (p->mode != GDPA_SCHED_FWD && p->mode != GDPA_SCHED_BWD && p->mode != GDPA_SCHED_FWD_SHARED_KV) return GDPA_ERR_BAD_ARG;
+  if (p->mode == GDPA_SCHED_FWD_SHARED_KV && p->kv_seq_index == nullptr) return GDPA_ERR_BAD_ARG;
   if (p->batch > 0 && (p->q_offsets == nullptr || p->kv_offsets == nullptr)) return GDPA_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(p->schedule) & 15u) != 0) return GDPA_ERR_MISALIGNED;
   if (p->schedule_bytes < kSchedHeaderInts * 4 + 16) return GDPA_ERR_CAPACITY;

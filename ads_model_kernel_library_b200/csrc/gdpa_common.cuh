@@ -8,7 +8,10 @@ namespace gdpa {
 
 constexpr int kTile = 128;          // rows of one Q tile / KV tile
 constexpr int kFwdQBlock = 256;     // Q rows of one forward work item (two Q tiles)
-constexpr int kSchedHeaderInts = 4; // schedule buffer: int32 header, then int4 work items
+constexpr int kSchedHeaderInts = 4; // schedule buffer: int32 header {count, mode, needed, counter}, then int4 work items
+// modes of a schedule; items {sequence, head, block, weight}, with kSchedFwdShared {first sequence of a run, head, first
+// row of the run this item takes, row past its last}
+constexpr int kSchedFwd = 0, kSchedBwd = 1, kSchedFwdShared = 2;
 
 // Activation classes the kernels are specialised on (several reference names share one class).
 enum ActClass : int {

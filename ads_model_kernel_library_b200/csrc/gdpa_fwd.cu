@@ -175,12 +175,12 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
   // ahead of its use; the MMA thread and the activation warps start on an item with two or three shared-memory loads
   // instead of making those trips each.  FP8 forward 4.96 -> 4.83 ms, the norm pipeline's step 7.77 -> 7.71 ms, the plain
   // forward of long and short items unchanged.
-  // Slot: {head, Q block, first Q row, first KV row}, {lq, lkv, first KV tile, KV tiles}, {Q scale row of Q tile 0, KV
+  // Slot: {head, row offset q0 of the Q block, first Q row, first KV row}, {lq, lkv, first KV tile, KV tiles}, {Q scale row of Q tile 0, KV
   // scale row of KV tile 0 (FP8), -, -}; head -1 ends the walk.
   int4* const work_ring = reinterpret_cast<int4*>(smem + L::kWorkOff);
   uint32_t work_pos = 0;  // items this role has taken: ring slot = work_pos % kWorkSlots, parity = (work_pos / kWorkSlots) & 1
   struct Item {
-    int h, blk, q_start, kv_start, lq, lkv, j0, nkv, q_scale0, kv_scale0;
+    int h, q0, q_start, kv_start, lq, lkv, j0, nkv, q_scale0, kv_scale0;  // the block takes rows [q0, min(lq, q0 + 256))
   };
   // Consumer side: this role's next work item; h = -1 at the end of the list, -2 if the wait ran out.
   // `warp_wide`: called by a whole warp, whose lane 0 releases the slot.
@@ -231,7 +231,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
           if (!__all_sync(0xffffffffu, ok)) return false;
           tmp_phase ^= 1u;
           for (int bx = 0; bx < L::kBoxes; ++bx)
-            for (int off = valid * 128 + lane * 16; off < L::kHalfBytes; off += 512)
+            for (int off = max(valid, 0) * 128 + lane * 16; off < L::kHalfBytes; off += 512)
               *reinterpret_cast<uint4*>(smem + dst_off + bx * L::kHalfBytes + off) = make_uint4(0, 0, 0, 0);
           fence_proxy_async_smem();
           __syncwarp();
@@ -240,6 +240,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         return true;
       };
       WorkWalker walker(n_items);
+      const bool shared_runs = a.sched[1] == kSchedFwdShared;
       // producer side of the work ring: the slot must have been read by every consumer of its previous use
       auto next_item = [&](Item& it) -> bool {
         const uint32_t slot = work_pos % kWorkSlots, parity = (work_pos / kWorkSlots) & 1u;
@@ -247,10 +248,16 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         int i;
         if (walker.next(i)) {
           const Work w = load_work(a.sched, i, a.q_off, a.kv_off, a.off64, a.max_q, a.max_kv, lim, a.kv_index);
-          it.h = w.h, it.blk = w.blk;
+          it.h = w.h, it.q0 = w.blk * kFwdQBlock;
           it.q_start = static_cast<int>(w.q_start), it.kv_start = static_cast<int>(w.kv_start);
           it.lq = w.lq, it.lkv = w.lkv;
           fwd_kv_range(w, a.window, it.j0, it.nkv);
+          if (shared_runs) {
+            // rows of a run of sequences instead of a block of one, still clamped to the tensor
+            const int4 run = reinterpret_cast<const int4*>(a.sched + kSchedHeaderInts)[i];
+            it.q0 = run.z;
+            it.lq = static_cast<int>(min(static_cast<long long>(run.w), a.total_q - w.q_start));
+          }
           if constexpr (FP8) {
             it.q_scale0 = static_cast<int>(load_offset(a.q_blk_off, w.b, a.off64)) + w.blk * 2;
             it.kv_scale0 = static_cast<int>(load_offset(a.kv_blk_off, w.kb, a.off64));
@@ -260,7 +267,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
                                   ((B_WORK_EMPTY + slot) << 8) | ST_ROLE_LOAD);
         if (!__all_sync(0xffffffffu, ok)) return false;
         if (lane == 0) {
-          work_ring[3 * slot] = make_int4(it.h, it.blk, it.q_start, it.kv_start);
+          work_ring[3 * slot] = make_int4(it.h, it.q0, it.q_start, it.kv_start);
           work_ring[3 * slot + 1] = make_int4(it.lq, it.lkv, it.j0, it.nkv);
           if (FP8) work_ring[3 * slot + 2] = make_int4(it.q_scale0, it.kv_scale0, 0, 0);
           mbar_arrive(bar_base + 8u * (B_WORK_FULL + slot));
@@ -274,7 +281,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         if (!next_item(w_next)) goto role_done;
         const int j0 = w.j0, nkv = w.nkv;  // first KV tile and number of KV tiles this item visits
         if (nkv == 0) continue;
-        const int q0 = w.blk * kFwdQBlock;
+        const int q0 = w.q0;
         const int nst = (w.lq - q0 > kTile) ? 2 : 1;
         const int q_row = w.q_start + q0;
         const int kv_row = w.kv_start + j0 * kTile;
@@ -351,7 +358,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         }
         const int nkv = w.nkv;
         if (nkv == 0) continue;
-        const int nst = (w.lq - w.blk * kFwdQBlock > kTile) ? 2 : 1;
+        const int nst = (w.lq - w.q0 > kTile) ? 2 : 1;
         // First S tiles: S_s = Q_s K_0^T.
         {
           const uint32_t k_stage = kv_stage;
@@ -423,7 +430,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         break;
       }
       const int j0 = w.j0, nkv = w.nkv;
-      const int q0 = w.blk * kFwdQBlock;
+      const int q0 = w.q0;
       const int nst = (w.lq - q0 > kTile) ? 2 : 1;
       if (s >= nst) continue;
       const int qr = q0 + s * kTile + row;
@@ -500,10 +507,10 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
             if (ch == 0) tmem_ld32(s_tmem + 32, rb);
             // a chunk wholly inside [clo, chi) for every row of the warp needs no predicates; without a band
             // the lower bound is 0
-            // (scale >= 0: the largest c * S is c times the largest S, one three-way maximum per two columns; with the
+            // (c >= 0: the largest c * S is c times the largest S, one three-way maximum per two columns; with the
             // packed arithmetic of pass 2 about 190 instead of 350 issue slots per warp and tile: FP8 forward 5.11 -> 4.96 ms,
             // bf16 training step 1.96 -> 1.94 ms)
-            if (a.scale >= 0.f && __all_sync(0xffffffffu, clo <= ch * 32 && chi >= (ch + 1) * 32)) {
+            if (c >= 0.f && __all_sync(0xffffffffu, clo <= ch * 32 && chi >= (ch + 1) * 32)) {
               float m0 = __uint_as_float(cur[0]), m1 = __uint_as_float(cur[1]);
 #pragma unroll
               for (int i = 2; i < 32; i += 4) {

@@ -4,7 +4,8 @@
 // sequence; backward items are (sequence, head, 128-row KV tile) weighted by the number of Q tiles.
 // The list is a counting sort by weight, heaviest first, built by one thread block without any
 // host synchronisation.  Buffer layout: int32 header {count, mode, 0, 0}, then one int4
-// {sequence, head, block, weight} per item.
+// {sequence, head, block, weight} per item ({first sequence, head, first row, row past the last} with kSchedFwdShared,
+// where neighbouring Q sequences of one KV sequence are taken together).
 #include "gdpa_common.cuh"
 #include "gdpa_launch.h"
 
@@ -14,6 +15,7 @@ namespace {
 
 constexpr int kSchedThreads = 1024;
 constexpr int kBins = 4096;
+constexpr int kSms = 148;  // CTAs of the persistent kernels
 
 __device__ __forceinline__ void seq_geometry(const SchedArgs& a, int b, int& nblk, int& weight) {
   long long s0, e0;
@@ -30,7 +32,7 @@ __device__ __forceinline__ void seq_geometry(const SchedArgs& a, int b, int& nbl
   lkv = lkv < 0 ? 0 : (lkv < a.max_kv ? lkv : a.max_kv);
   const int nq = static_cast<int>((lq + kTile - 1) / kTile);
   const int nkv = static_cast<int>((lkv + kTile - 1) / kTile);
-  if (a.mode == 0) {
+  if (a.mode != kSchedBwd) {
     nblk = static_cast<int>((lq + kFwdQBlock - 1) / kFwdQBlock);
     weight = nkv;
   } else {
@@ -40,27 +42,86 @@ __device__ __forceinline__ void seq_geometry(const SchedArgs& a, int b, int& nbl
   if (weight > kBins - 1) weight = kBins - 1;
 }
 
+// The same for kSchedFwdShared, for the 1024 sequences from b0: sequences that follow one another, read the same KV
+// sequence and are not cut by max_q form a run, one long sequence as far as the forward is concerned (their rows are
+// neighbours in the packed tensors).  The first sequence of a run gets all its blocks, the others none; runs end at the
+// end of a chunk.  (4 requests of 64 candidates of 1 to 32 rows, 4 heads: 1 024 items of one mostly empty Q tile became 140
+// full ones, the forward kernel 75 -> 20 us.)  Called by the whole block; `first_head[w]` is the first run head among warp w's sequences.
+__device__ __forceinline__ void run_geometry(const SchedArgs& a, int b0, int n, int piece, int* first_head, int& nblk, int& weight,
+                                             int& rows) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int b = b0 + t;
+  auto kv_of = [&](int i) {
+    const int kb = static_cast<int>(load_offset(a.kv_index, i, a.off64));
+    return kb < 0 ? 0 : (kb >= a.kv_batch ? a.kv_batch - 1 : kb);
+  };
+  auto whole = [&](int i) {
+    const long long len = load_offset(a.q_off, i + 1, a.off64) - load_offset(a.q_off, i, a.off64);
+    return len >= 0 && len <= a.max_q;
+  };
+  const bool joins = t < n && whole(b);
+  const bool head = t < n && (t == 0 || !joins || !whole(b - 1) || kv_of(b) != kv_of(b - 1));
+  const unsigned heads = __ballot_sync(0xffffffffu, head);
+  if (lane == 0) first_head[warp] = heads != 0u ? warp * 32 + __ffs(heads) - 1 : -1;
+  __syncthreads();
+  nblk = 0, weight = 0, rows = 0;
+  if (head) {
+    seq_geometry(a, b, nblk, weight);  // the weight; the blocks follow from the rows of the run
+    long long s0, e0;
+    seq_bounds(a.q_off, b, a.off64, s0, e0);
+    long long len = e0 - s0;
+    if (joins) {
+      int end = n;  // of the run, within the chunk
+      const unsigned later = lane < 31 ? heads >> (lane + 1) : 0u;
+      if (later != 0u) {
+        end = t + __ffs(later);
+      } else {
+        for (int w = warp + 1; w < kSchedThreads / 32; ++w)
+          if (first_head[w] >= 0) {
+            end = first_head[w];
+            break;
+          }
+      }
+      len = load_offset(a.q_off, b0 + end, a.off64) - s0;
+    } else {
+      len = len < 0 ? 0 : a.max_q;
+    }
+    rows = static_cast<int>(len);
+    nblk = (rows + piece - 1) / piece;
+  }
+  __syncthreads();  // first_head is written again by the next call
+}
+
 // Latency-bound: one block, a few thousand items, and the forward or backward kernel waits for it.  What it costs is the
 // chain of dependent steps, so: only the bins that a sequence of the given maximum length can have are cleared and
 // scanned (17 of 4096 for 2048 tokens), the scan gives each thread its own run of neighbouring bins (a warp reads
 // consecutive words, no bank conflicts) instead of one warp walking all of them, and the items of a chunk of 1024
 // sequences are written by all warps together, 32 consecutive items (512 bytes) per store, instead of each thread
-// writing the items of one sequence one after another (13 us for 8 sequences, 26 us for 1024, a call of 256 short
-// sequences 86.7 -> 81.8 us in all).
+// writing the items of one sequence one after another (13 -> 4 us for 8 sequences, 26 -> 15 us for 1024).
 __global__ void __launch_bounds__(kSchedThreads, 1) gdpa_build_schedule_kernel(const SchedArgs a) {
   __shared__ int hist[kBins];
   __shared__ int warp_sum[kSchedThreads / 32];
-  __shared__ int4 seq[kSchedThreads];  // of the sequences of one chunk: first slot, blocks, weight, -
+  __shared__ int4 seq[kSchedThreads];  // of the sequences of one chunk: first slot, blocks, weight, rows (of a run)
+  __shared__ int first_head[kSchedThreads / 32];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int longest = a.mode == 0 ? a.max_kv : a.max_q;
+  const bool shared = a.mode == kSchedFwdShared;
+  const int longest = a.mode == kSchedBwd ? a.max_q : a.max_kv;
   const int bins = min(kBins, (longest > 0 ? (longest - 1) / kTile + 1 : 0) + 1);  // weights 0 .. bins - 1
   const long long cap = a.capacity_items;
   for (int i = t; i < bins; i += kSchedThreads) hist[i] = 0;
   __syncthreads();
-  int nblk = 0, w = 0;  // of this thread's sequence of the last chunk: the only one unless the batch is large
-  for (int b = t; b < a.batch; b += kSchedThreads) {
-    seq_geometry(a, b, nblk, w);
-    if (nblk > 0) atomicAdd(&hist[w], nblk * a.heads);
+  // Runs are cut into blocks of two Q tiles when that gives every CTA one, else of one tile: with idle CTAs the longest
+  // block is what the call takes, and one tile is done sooner than two.
+  int piece = kFwdQBlock;
+  if (shared && a.batch > 0 &&
+      (load_offset(a.q_off, a.batch, a.off64) - load_offset(a.q_off, 0, a.off64)) / kFwdQBlock * a.heads < kSms)
+    piece = kTile;
+  int nblk = 0, w = 0, rows = 0;  // of this thread's sequence of the last chunk: the only one unless the batch is large
+  for (int b0 = 0; b0 < a.batch; b0 += kSchedThreads) {
+    const int n = min(kSchedThreads, a.batch - b0);
+    if (shared) run_geometry(a, b0, n, piece, first_head, nblk, w, rows);
+    else if (t < n) seq_geometry(a, b0 + t, nblk, w);
+    if (t < n && nblk > 0) atomicAdd(&hist[w], nblk * a.heads);
   }
   __syncthreads();
   // Exclusive prefix over bins from the heaviest down: hist[w] becomes the first slot of weight w.  Thread t owns the
@@ -97,10 +158,13 @@ __global__ void __launch_bounds__(kSchedThreads, 1) gdpa_build_schedule_kernel(c
   int4* items = reinterpret_cast<int4*>(a.sched + kSchedHeaderInts);
   for (int b0 = 0; b0 < a.batch; b0 += kSchedThreads) {
     const int n = min(kSchedThreads, a.batch - b0);
+    if (a.batch > kSchedThreads) {
+      if (shared) run_geometry(a, b0, n, piece, first_head, nblk, w, rows);
+      else if (t < n) seq_geometry(a, b0 + t, nblk, w);
+    }
     if (t < n) {
-      if (a.batch > kSchedThreads) seq_geometry(a, b0 + t, nblk, w);
       const int count = nblk * a.heads;
-      seq[t] = make_int4(count > 0 ? atomicAdd(&hist[w], count) : 0, nblk, w, 0);
+      seq[t] = make_int4(count > 0 ? atomicAdd(&hist[w], count) : 0, nblk, w, rows);
     }
     __syncthreads();
     for (int i = warp; i < n; i += kSchedThreads / 32) {
@@ -108,8 +172,9 @@ __global__ void __launch_bounds__(kSchedThreads, 1) gdpa_build_schedule_kernel(c
       const int count = sq.y * a.heads;
       for (int k = lane; k < count; k += 32) {
         const long long slot = static_cast<long long>(sq.x) + k;
-        const int h = k / sq.y;
-        if (slot < cap) items[slot] = make_int4(b0 + i, h, k - h * sq.y, sq.z);
+        const int h = k / sq.y, blk = k - h * sq.y;
+        if (slot < cap)
+          items[slot] = shared ? make_int4(b0 + i, h, blk * piece, min(sq.w, (blk + 1) * piece)) : make_int4(b0 + i, h, blk, sq.z);
       }
     }
     __syncthreads();

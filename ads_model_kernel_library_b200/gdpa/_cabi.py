@@ -20,6 +20,7 @@ GDPA_DTYPE_FP8_E4M3 = 1
 GDPA_OFFSETS_INT64, GDPA_OFFSETS_PAIRS = 1, 2
 GDPA_SCHED_FWD = 0
 GDPA_SCHED_BWD = 1
+GDPA_SCHED_FWD_SHARED_KV = 2
 GDPA_ACT_SOFTMAX = 100
 
 EXPORTS = (

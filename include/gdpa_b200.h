@@ -89,7 +89,12 @@ enum { GDPA_DTYPE_BF16 = 0, GDPA_DTYPE_FP8_E4M3 = 1 };
 /* Which pass a schedule is for. */
 enum {
   GDPA_SCHED_FWD = 0, /* one work item per (sequence, head, 256-row Q block)  */
-  GDPA_SCHED_BWD = 1  /* one work item per (sequence, head, 128-row KV tile)  */
+  GDPA_SCHED_BWD = 1, /* one work item per (sequence, head, 128-row KV tile)  */
+  /* Forward with kv_seq_index and no window: neighbouring Q sequences that read the same KV sequence are taken
+   * together, one work item per (run of sequences, head, 256- or 128-row Q block).  For gdpa_fwd only (not for
+   * gdpa_fwd_fp8, whose scales are per sequence, and not for a call with a window, which counts positions in the
+   * sequence). */
+  GDPA_SCHED_FWD_SHARED_KV = 2
 };
 
 /* ---------------------------------------------------------------------------------------------
@@ -100,7 +105,7 @@ enum {
  * ------------------------------------------------------------------------------------------- */
 typedef struct GdpaSchedParams {
   uint32_t struct_size;       /* sizeof(GdpaSchedParams) */
-  int32_t mode;               /* GDPA_SCHED_FWD or GDPA_SCHED_BWD */
+  int32_t mode;               /* GDPA_SCHED_* */
   const void* q_offsets;      /* [batch + 1] */
   const void* kv_offsets;     /* [batch + 1] */
   int32_t offsets_are_int64;
@@ -119,7 +124,7 @@ typedef struct GdpaSchedParams {
 } GdpaSchedParams;
 
 /* Bytes needed for a schedule of the given pass.  total_rows is total_q for GDPA_SCHED_FWD and
- * total_kv for GDPA_SCHED_BWD.  Pure host arithmetic. */
+ * total_kv for GDPA_SCHED_BWD, total_q for GDPA_SCHED_FWD_SHARED_KV.  Pure host arithmetic. */
 size_t gdpa_schedule_bytes(int32_t mode, int64_t total_rows, int32_t batch, int32_t heads);
 
 /* Build the schedule on `stream`.  No host synchronisation. */

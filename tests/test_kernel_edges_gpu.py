@@ -123,3 +123,55 @@ def test_softmax_forward_for_every_sign_of_the_scale(D, scale):
         qb, (kb, vb) = q[qo[b]:qo[b + 1]].double(), (t[ko[b]:ko[b + 1]].double() for t in (k, v))
         p = torch.softmax(torch.einsum("qhd,khd->hqk", qb, kb) * scale, -1)
         assert_close(o[qo[b]:qo[b + 1]], torch.einsum("hqk,khd->qhd", p, vb), f"O[{lq[b]}, {lk[b]}]")
+
+
+@pytest.mark.parametrize("requests,per,rows,heads", [(1, 5, 9, 1), (3, 64, 32, 2), (2, 700, 60, 2), (40, 33, 200, 2)])
+def test_shared_kv_runs_cover_every_row_once(requests, per, rows, heads):
+    """Sequences of one KV sequence are scheduled together, in blocks of 128 rows for few rows and 256 for many; a
+    sequence longer than the maximum is cut, entries beyond the KV batch are clamped, empty sequences take no rows."""
+    rng = np.random.default_rng(per)
+    batch = requests * per
+    lq = rng.integers(0, rows + 1, batch)
+    if rows > 100:
+        lq[batch // 2] = rows + 50  # cut at max_q
+    index = np.repeat(np.arange(requests), per)
+    index[-1] = requests + 3  # clamped to the last request
+    index[per // 2] = requests - 1  # breaks a run
+    lk = rng.integers(1, 900, requests)
+    qo, ko, idx = torch.tensor(np.concatenate([[0], np.cumsum(lq)])).cuda(), torch.tensor(np.concatenate([[0], np.cumsum(lk)])).cuda(), \
+        torch.tensor(index).cuda()
+    header, items = _schedule(qo, ko, 2, heads, rows, 1000, idx)
+    assert header[0] == header[2] == len(items)
+    owner = np.full((heads, int(qo[-1])), -1)
+    start = qo.cpu().numpy()
+    for b, h, first, end in items.tolist():
+        assert first < end <= first + 256
+        at = owner[h, start[b] + first:start[b] + end]
+        assert (at == -1).all() and len(at) == end - first
+        at[:] = min(index[b], requests - 1)
+    for b in range(batch):
+        n = min(lq[b], rows)
+        assert (owner[:, start[b]:start[b] + n] == min(index[b], requests - 1)).all()
+        assert (owner[:, start[b] + n:start[b + 1]] == -1).all()
+
+
+@pytest.mark.parametrize("D,act", [(64, "silu"), (128, "gelu_approx"), (128, "softmax")])
+@pytest.mark.parametrize("per,rows", [(7, 20), (150, 90)])
+def test_shared_kv_runs_give_what_single_sequences_give(G, D, act, per, rows):
+    """The same call with a band that reaches every pair is scheduled sequence by sequence.  Same products; the fp32 sums
+    may be split over the two accumulators differently (some 1e-7 of the sum of at most 700 terms of a few units: 1e-3),
+    and one that lies near a rounding boundary then differs by an ulp of bf16, 2^-7.  (Softmax: when a row's running
+    maximum moves depends on the rows beside it, so its P is rounded to bf16 from another base, a few such ulps.)"""
+    g = torch.Generator().manual_seed(per)
+    rng = np.random.default_rng(per)
+    requests, H = 3, 2
+    lq, lk = rng.integers(0, rows + 1, requests * per), rng.integers(1, 700, requests)
+    qo, ko = (torch.tensor(np.concatenate([[0], np.cumsum(n)])).cuda() for n in (lq, lk))
+    q = torch.randn(int(qo[-1]), H, D, generator=g).to(torch.bfloat16).cuda()
+    k, v = (torch.randn(int(ko[-1]), H, D, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    index = torch.arange(requests).repeat_interleave(per).cuda()
+    out = [G.generalized_dot_product_attention(q, k, v, qo, ko, rows, 700, ad_to_request_offset=index, qk_scale=0.1, activation=act,
+                                               window_size=w) for w in (None, 1 << 20)]
+    torch.cuda.synchronize()
+    assert G.kernel_status() == 0
+    assert_close(out[0], out[1], "runs", atol=1e-2 if act == "softmax" else 1e-3, rtol=1e-2 if act == "softmax" else 2.0 ** -7)
