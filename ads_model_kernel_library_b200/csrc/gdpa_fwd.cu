@@ -470,11 +470,13 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         float* rowmax = reinterpret_cast<float*>(smem + L::kRowMaxOff);
         float* rowsum = reinterpret_cast<float*>(smem + L::kRowSumOff);
         float m_used = -INFINITY, row_sum = 0.f;
-        float sq = 1.f;
-        long long kv_blk0 = 0;
+        float sq = 1.f, sk_next = 1.f, sv_next = 1.f;
+        const float *k_scale = nullptr, *v_scale = nullptr;
         if constexpr (FP8) {
           sq = a.q_scales[static_cast<long long>(w.q_scale0 + s) * a.heads + w.h];
-          kv_blk0 = w.kv_scale0;
+          const long long at = static_cast<long long>(w.kv_scale0 + j0) * a.kv_heads + w.h / a.kv_group;
+          k_scale = a.k_scales + at, v_scale = a.v_scales + at;
+          sk_next = *k_scale, sv_next = *v_scale;
         }
         for (int j = 0; j < nkv; ++j) {
           // columns [clo, chi) of this warp's 64 take part: inside the KV length and inside the band
@@ -486,11 +488,14 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
           }
           float c = a.scale * kLog2e, bias = 0.f, inv_sv = 1.f;
           if constexpr (FP8) {
-            const float sk = a.k_scales[(kv_blk0 + j0 + j) * a.kv_heads + w.h / a.kv_group];
-            const float sv = a.v_scales[(kv_blk0 + j0 + j) * a.kv_heads + w.h / a.kv_group];
-            c *= sq * sk;
-            bias = log2f(sv);
-            inv_sv = 1.f / sv;
+            // this tile's scales were asked for a tile ago
+            c *= sq * sk_next;
+            bias = log2f(sv_next);
+            inv_sv = 1.f / sv_next;
+            if (j + 1 < nkv) {
+              k_scale += a.kv_heads, v_scale += a.kv_heads;
+              sk_next = *k_scale, sv_next = *v_scale;
+            }
           }
           GDPA_WAIT_WARP(B_S_FULL + s, s_phase, ST_ROLE_ACT);
           tc_fence_after();
