@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+from oracle import gdpa_oracle as orc
 from tests._util import assert_close
 
 pytestmark = pytest.mark.gpu
@@ -175,3 +176,34 @@ def test_shared_kv_runs_give_what_single_sequences_give(G, D, act, per, rows):
     torch.cuda.synchronize()
     assert G.kernel_status() == 0
     assert_close(out[0], out[1], "runs", atol=1e-2 if act == "softmax" else 1e-3, rtol=1e-2 if act == "softmax" else 2.0 ** -7)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_fp8_quantiser_rounds_as_a_division(G, D):
+    """The one-pass quantiser against the restatement, byte for byte: ragged blocks, more sequences than one round of the
+    owner search holds, zeros, denormals, a block with an infinity, a NaN, and every bf16 mantissa over many scales."""
+    g = torch.Generator().manual_seed(D)
+    lens = [130, 0, 1, 128, 127, 384] + [5, 0, 3] * 20
+    off = torch.tensor(np.concatenate([[0], np.cumsum(lens)]))
+    T, H = int(off[-1]), 3
+    x = (torch.randn(T, H, D, generator=g) * torch.exp2(torch.randint(-30, 30, (T, H, 1), generator=g).float())).to(torch.bfloat16)
+    x[0:131, 0] = 0
+    x[131:140, 1] = 1e-39
+    x[260:300, 2, 3] = float("inf")
+    x8, sc, bo = G.quantize_fp8_blockwise(x.cuda(), off.cuda())
+    torch.cuda.synchronize()
+    r8, rsc, rbo = orc.quantize_fp8_blockwise(x, off)
+    assert torch.equal(bo.cpu(), rbo.to(bo.dtype)) and torch.equal(sc.cpu()[: rsc.shape[0]], rsc)
+    same = x8.cpu().view(torch.uint8) == r8.view(torch.uint8)
+    same |= ~torch.isfinite(x.float())  # inf / inf is a NaN: the restatement's clamp keeps it, the kernels give -448
+    assert same.all()
+    n = 1 << 20  # the quotients themselves, scales of every mantissa
+    amax = (torch.randint(0x3F80, 0x4000, (n // 128,), generator=g).to(torch.int16).view(torch.bfloat16)).float()
+    v = (torch.rand(n // 128, 128, generator=g) * 2 - 1) * amax[:, None]
+    v[:, 0] = amax
+    y = v.to(torch.bfloat16).view(-1, 1, 128)
+    yo = torch.arange(0, n // 128 + 1)  # one-row sequences: a scale per row
+    y8, _, _ = G.quantize_fp8_blockwise(y.cuda(), yo.cuda())
+    scale = (y.float().abs().amax(2, keepdim=True) / 448).clamp_min(1e-12)
+    want = (y.float() / scale).clamp(-448, 448).to(torch.float8_e4m3fn)
+    assert torch.equal(y8.cpu().view(torch.uint8), want.view(torch.uint8))
