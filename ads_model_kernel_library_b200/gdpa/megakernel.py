@@ -18,7 +18,7 @@ import torch
 
 from . import _cabi
 from .math import SOFTMAX_ID, activation_string_to_int
-from .ops import (_build_schedule, _check_inputs, _fill_fwd_params, _set_timing, _stream_ptr, expect_contiguous)
+from .ops import (_build_schedule, _check_inputs, _fill_fwd_params, _on_device, _set_timing, _stream_ptr, expect_contiguous)
 
 NORM_EPS = 1e-5
 
@@ -51,7 +51,7 @@ def layernorm_rows(x: torch.Tensor, weight: Optional[torch.Tensor] = None, bias:
     n = int(torch.Size(x.shape[1:]).numel())
     out = torch.empty_like(x)
     w, b = _vector(weight, n, "layernorm_weight", x.device), _vector(bias, n, "layernorm_bias", x.device)
-    with torch.cuda.device(x.device):
+    with _on_device(x):
         p = _norm_params(x, out, n, eps)
         p.weight = w.data_ptr() if w is not None else None
         p.bias = b.data_ptr() if b is not None else None
@@ -73,7 +73,7 @@ def rmsnorm_rows(x: torch.Tensor, weight: Optional[torch.Tensor] = None, residua
     w = _vector(weight, n, "rms_norm_weight", x.device)
     if residual is not None and (residual.shape != x.shape or residual.dtype != x.dtype or not residual.is_contiguous()):
         raise ValueError("residual must be a contiguous tensor of the shape and dtype of the output")
-    with torch.cuda.device(x.device):
+    with _on_device(x):
         p = _norm_params(x, out, n, eps)
         p.weight = w.data_ptr() if w is not None else None
         p.residual = residual.data_ptr() if residual is not None else None
@@ -93,7 +93,7 @@ def norm_rows_backward(mode: int, dy: torch.Tensor, dy_add: Optional[torch.Tenso
     w = _vector(weight, n, "weight", dy.device)
     dw = torch.zeros(n, dtype=torch.float32, device=dy.device) if want_dweight else None
     db = torch.zeros(n, dtype=torch.float32, device=dy.device) if want_dbias else None
-    with torch.cuda.device(dy.device):
+    with _on_device(dy):
         p = _cabi.GdpaNormBwdParams()
         p.struct_size = C.sizeof(_cabi.GdpaNormBwdParams)
         p.mode, p.rows, p.n = mode, dy.shape[0], n
@@ -138,7 +138,7 @@ def _gdpa_with_norms_op(
         raise ValueError("query must be contiguous for the norm pipeline")
     dev, T = query.device, query.shape[0]
     none = lambda dtype=torch.float32: torch.empty(0, dtype=dtype, device=dev)  # noqa: E731
-    with torch.cuda.device(dev):
+    with _on_device(query):
         keep_ln = fused_layernorm and save_for_backward
         ln_mean = torch.empty(T, dtype=torch.float32, device=dev) if keep_ln else none()
         ln_rstd = torch.empty(T, dtype=torch.float32, device=dev) if keep_ln else none()

@@ -20,7 +20,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _cabi
-from .ops import _stream_ptr, generalized_dot_product_attention
+from .ops import _on_device, _stream_ptr, generalized_dot_product_attention
 
 __all__ = ["quantize_varlen_mxfp8_sf_only", "dequantize_mxfp8", "generalized_dot_product_attention_mxfp8"]
 
@@ -89,7 +89,7 @@ def quantize_varlen_mxfp8_sf_only(
         sf_blocks = int(((lens + 127) // 128).sum())
     else:
         sf_blocks = total // 128 + batch
-    with torch.cuda.device(x.device):
+    with _on_device(x):
         x8 = torch.empty(x.shape, dtype=torch.float8_e4m3fn, device=x.device)
         sf = torch.zeros(_sf_shape(H, D, max(sf_blocks, 1), scale_axis), dtype=torch.uint8, device=x.device)
         blk_off = _run(True, x, x8, sf, cu_seqlens, scale_axis, max(sf_blocks, 1) if total > 0 else 0)
@@ -121,7 +121,7 @@ def dequantize_mxfp8(
     sf_blocks = sf.numel() // (H * d_atoms * 512)
     x8 = x8.contiguous()
     sf = sf.contiguous()
-    with torch.cuda.device(x8.device):
+    with _on_device(x8):
         out = torch.empty(x8.shape, dtype=dtype, device=x8.device)
         _run(False, out, x8, sf, cu_seqlens.contiguous(), scale_axis, sf_blocks)
     return out
