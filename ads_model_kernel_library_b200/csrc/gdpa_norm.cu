@@ -193,8 +193,8 @@ __global__ void __launch_bounds__(kNormThreads) gdpa_rmsnorm_rows_kernel(const N
 // columns in every row its group takes, so the weight and bias gradients (sums over rows) are plain register sums for
 // the whole kernel, added up over the block's groups in shared memory once at the end and flushed with one global
 // atomic per column and block.  Before, every value of every row was a shared-memory atomic and the row was read twice:
-// 543 us (RMS norm) and 957 us (layer norm) for 149 713 rows of 1024 (floors at the copy rate 138 and 184 us), and the
-// whole forward and backward of that pipeline took 8.52 ms against 7.66 ms with this kernel.
+// 543 us (RMS norm) and 957 us (layer norm) for 149 713 rows of 1024, now 188 and 257 us (floors at the copy rate 138 and
+// 184 us); the whole forward and backward of that pipeline 8.52 -> 7.66 ms.
 // Two chunks per lane keep the kernel under 80 (RMS norm) and 128 registers (layer norm), so three and two blocks of
 // eight warps are resident and 48 KB of loads are in flight per SM.
 constexpr int kNormBwdMaxN = 4096;  // 8 warps x 32 lanes x 2 chunks x 8 values; the gradients of w and b end there too

@@ -46,7 +46,7 @@ __device__ __forceinline__ void seq_geometry(const SchedArgs& a, int b, int& nbl
 // sequence and are not cut by max_q form a run, one long sequence as far as the forward is concerned (their rows are
 // neighbours in the packed tensors).  The first sequence of a run gets all its blocks, the others none; runs end at the
 // end of a chunk.  (4 requests of 64 candidates of 1 to 32 rows, 4 heads: 1 024 items of one mostly empty Q tile became 140
-// full ones, the forward kernel 75 -> 20 us.)  Called by the whole block; `first_head[w]` is the first run head among warp w's sequences.
+// full ones, the forward kernel 75 -> 23 us.)  Called by the whole block; `first_head[w]` is the first run head among warp w's sequences.
 __device__ __forceinline__ void run_geometry(const SchedArgs& a, int b0, int n, int piece, int* first_head, int& nblk, int& weight,
                                              int& rows) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
