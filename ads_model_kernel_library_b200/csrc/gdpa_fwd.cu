@@ -55,10 +55,10 @@ enum FwdBar : int {
   B_O_EMPTY = 10 + 2 * kKvStages,      // [2] epilogue (256 arrivals) -> MMA
   B_L_FULL = 12 + 2 * kKvStages,       // [2] softmax: activation group -> epilogue (row sums)
   B_M_FULL = 14 + 2 * kKvStages,       // [2] softmax, wide layout: both column halves have published their row maxima
-  B_LD_TMP = 16 + 2 * kKvStages,       // the loader's own: a ragged tile has landed and can have its padding rows zeroed
-  B_WORK_FULL = 17 + 2 * kKvStages,               // [kWorkSlots] the loader has published a work item
-  B_WORK_EMPTY = 17 + 2 * kKvStages + kWorkSlots, // [kWorkSlots] the MMA thread and the 16 activation warps have read it
-  B_COUNT = 17 + 2 * kKvStages + 2 * kWorkSlots
+  B_LD_TMP = 16 + 2 * kKvStages,       // [4] the loader's own: a ragged tile has landed and can have its padding rows zeroed
+  B_WORK_FULL = 20 + 2 * kKvStages,               // [kWorkSlots] the loader has published a work item
+  B_WORK_EMPTY = 20 + 2 * kKvStages + kWorkSlots, // [kWorkSlots] the MMA thread and the 16 activation warps have read it
+  B_COUNT = 20 + 2 * kKvStages + 2 * kWorkSlots
 };
 
 template <int D, int EB>
@@ -214,29 +214,32 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
     // the warp overwrites those rows with zeros in shared memory and only then releases the tile: the consumers see a
     // zero-padded tile and nothing of the neighbour reaches them.
     {
-      uint32_t kv_stage = 0, kv_phase = 0, q_phase = 0, tmp_phase = 0;  // bit s of q_phase = parity of Q stage s
+      uint32_t kv_pos = 0;  // K / V tiles of the items before this one; tile number p sits in ring slot p % kKvStages
+      uint32_t q_phase = 0, tmp_phase = 0;  // bit s = parity of Q stage s, of B_LD_TMP + s
       [[maybe_unused]] int ltr = 0;  // KV tiles before this item (trace rows)
-      // one tile = L::kBoxes boxes of 128 rows x 128 bytes; `ragged`: onto the loader's barrier, then zero rows >= valid
-      auto load_tile = [&](uint32_t dst_off, const CUtensorMap* tm, int full_bar, int y, int row0, int valid) -> bool {
-        const bool ragged = valid < kTile;
+      // asks for one tile = L::kBoxes boxes of 128 rows x 128 bytes; a ragged one (valid < 128) on B_LD_TMP + tmp
+      auto load_tile = [&](uint32_t dst_off, const CUtensorMap* tm, int full_bar, int tmp, int y, int row0, int valid) {
         if (lane == 0) {
-          const uint32_t bar = bar_base + 8u * (ragged ? B_LD_TMP : full_bar);
+          const uint32_t bar = bar_base + 8u * (valid < kTile ? B_LD_TMP + tmp : full_bar);
           mbar_arrive_expect_tx(bar, L::kTileBytes);
 #pragma unroll
           for (int hf = 0; hf < L::kBoxes; ++hf)
             tma_load_3d(smem_base + dst_off + hf * L::kHalfBytes, tm, bar, hf * L::kBoxCols, y, row0);
         }
-        if (ragged) {
-          const bool ok = mbar_wait(bar_base + 8u * B_LD_TMP, tmp_phase, abort_flag, a.status, (B_LD_TMP << 8) | ST_ROLE_LOAD);
-          if (!__all_sync(0xffffffffu, ok)) return false;
-          tmp_phase ^= 1u;
-          for (int bx = 0; bx < L::kBoxes; ++bx)
-            for (int off = max(valid, 0) * 128 + lane * 16; off < L::kHalfBytes; off += 512)
-              *reinterpret_cast<uint4*>(smem + dst_off + bx * L::kHalfBytes + off) = make_uint4(0, 0, 0, 0);
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_base + 8u * full_bar);
-        }
+      };
+      // a ragged tile: once it has landed, zero its rows >= valid and release it on its consumers' barrier
+      auto release = [&](uint32_t dst_off, int full_bar, int tmp, int valid) -> bool {
+        if (valid >= kTile) return true;
+        const bool ok = mbar_wait(bar_base + 8u * (B_LD_TMP + tmp), (tmp_phase >> tmp) & 1u, abort_flag, a.status,
+                                  ((B_LD_TMP + tmp) << 8) | ST_ROLE_LOAD);
+        if (!__all_sync(0xffffffffu, ok)) return false;
+        tmp_phase ^= 1u << tmp;
+        for (int bx = 0; bx < L::kBoxes; ++bx)
+          for (int off = max(valid, 0) * 128 + lane * 16; off < L::kHalfBytes; off += 512)
+            *reinterpret_cast<uint4*>(smem + dst_off + bx * L::kHalfBytes + off) = make_uint4(0, 0, 0, 0);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_base + 8u * full_bar);
         return true;
       };
       WorkWalker walker(n_items);
@@ -285,30 +288,45 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         const int nst = (w.lq - q0 > kTile) ? 2 : 1;
         const int q_row = w.q_start + q0;
         const int kv_row = w.kv_start + j0 * kTile;
-        // Issue order Q0, K0, Q1, V0, K1, V1, ...
-        for (int step = 0; step < 2 * nkv + 2; ++step) {
-          if (step == 0 || step == 2) {
-            const int s = step >> 1;
-            if (s >= nst) continue;
-            if (lane == 0) GDPA_TRACE(a, ltr * 32 + 24 + s * 2);
-            GDPA_WAIT_WARP(B_Q_EMPTY + s, ((q_phase >> s) & 1u) ^ 1u, ST_ROLE_LOAD);
-            if (lane == 0) GDPA_TRACE(a, ltr * 32 + 25 + s * 2);
-            q_phase ^= 1u << s;
-            if (!load_tile(L::kQOff + s * L::kTileBytes, &tm_q.m[0], B_Q_FULL + s, w.h, q_row + s * kTile,
-                           w.lq - q0 - s * kTile))
-              goto role_done;
-          } else {
-            const int t = (step == 1) ? 0 : step - 2;  // 0 = K0, 1 = V0, 2 = K1, ...
-            const int j = t >> 1;
-            GDPA_WAIT_WARP(B_KV_EMPTY + kv_stage, kv_phase ^ 1u, ST_ROLE_LOAD);
-            if (!load_tile(L::kKvOff + kv_stage * L::kTileBytes, (t & 1) ? &tm_v.m[0] : &tm_k.m[0], B_KV_FULL + kv_stage,
-                           w.h / a.kv_group, kv_row + j * kTile, w.lkv - (j0 + j) * kTile))
-              goto role_done;
-            if (++kv_stage == kKvStages) {
-              kv_stage = 0;
-              kv_phase ^= 1u;
-            }
+        // Issue order Q0, K0, Q1, V0, K1, V1, ...  In an item of one or two KV tiles (all its tiles fit in the ring) none of
+        // the copies of a group (the first four, then K1 and V1) waits for another to land: ragged tiles are zeroed and
+        // released when the whole group has been asked for.  There the round trips to memory are what the item takes
+        // (training on lengths up to 256: 801 -> 755 us, the forward kernel 204 -> 162 us); with more KV tiles the loader is
+        // ahead of the MMAs, and a ragged K that waits for the ring slot of its V would come later than it could (log-normal
+        // forward 1.215 -> 1.232 ms with groups everywhere).  The softmax kernels' items are bound by their element-wise
+        // work: FP8 4.82 -> 4.86 ms with groups, so they have none.
+        const bool group = !kSoftmax && nkv <= 2;
+        const int head_kv = w.h / a.kv_group;
+        const int q_valid0 = w.lq - q0, q_valid1 = w.lq - q0 - kTile;
+        for (int j = 0; j < nkv; ++j) {
+          const int kv_valid = w.lkv - (j0 + j) * kTile;
+          const uint32_t k_stage = kv_pos % kKvStages, v_stage = (kv_pos + 1) % kKvStages;
+          const uint32_t k_off = L::kKvOff + k_stage * L::kTileBytes, v_off = L::kKvOff + v_stage * L::kTileBytes;
+          if (j == 0) {
+            if (lane == 0) GDPA_TRACE(a, ltr * 32 + 24);
+            GDPA_WAIT_WARP(B_Q_EMPTY, (q_phase & 1u) ^ 1u, ST_ROLE_LOAD);
+            q_phase ^= 1u;
+            load_tile(L::kQOff, &tm_q.m[0], B_Q_FULL, 0, w.h, q_row, q_valid0);
+            if (!group && !release(L::kQOff, B_Q_FULL, 0, q_valid0)) goto role_done;
           }
+          GDPA_WAIT_WARP(B_KV_EMPTY + k_stage, ((kv_pos / kKvStages) & 1u) ^ 1u, ST_ROLE_LOAD);
+          load_tile(k_off, &tm_k.m[0], B_KV_FULL + k_stage, 2, head_kv, kv_row + j * kTile, kv_valid);
+          if (!group && !release(k_off, B_KV_FULL + k_stage, 2, kv_valid)) goto role_done;
+          if (j == 0 && nst == 2) {
+            GDPA_WAIT_WARP(B_Q_EMPTY + 1, ((q_phase >> 1) & 1u) ^ 1u, ST_ROLE_LOAD);
+            q_phase ^= 2u;
+            load_tile(L::kQOff + L::kTileBytes, &tm_q.m[0], B_Q_FULL + 1, 1, w.h, q_row + kTile, q_valid1);
+            if (!group && !release(L::kQOff + L::kTileBytes, B_Q_FULL + 1, 1, q_valid1)) goto role_done;
+          }
+          GDPA_WAIT_WARP(B_KV_EMPTY + v_stage, (((kv_pos + 1) / kKvStages) & 1u) ^ 1u, ST_ROLE_LOAD);
+          load_tile(v_off, &tm_v.m[0], B_KV_FULL + v_stage, 3, head_kv, kv_row + j * kTile, kv_valid);
+          if (group) {
+            if (j == 0 && !release(L::kQOff, B_Q_FULL, 0, q_valid0)) goto role_done;
+            if (!release(k_off, B_KV_FULL + k_stage, 2, kv_valid)) goto role_done;
+            if (j == 0 && nst == 2 && !release(L::kQOff + L::kTileBytes, B_Q_FULL + 1, 1, q_valid1)) goto role_done;
+          }
+          if (!release(v_off, B_KV_FULL + v_stage, 3, kv_valid)) goto role_done;
+          kv_pos += 2;
         }
         ltr += nkv;
       }

@@ -207,3 +207,25 @@ def test_fp8_quantiser_rounds_as_a_division(G, D):
     scale = (y.float().abs().amax(2, keepdim=True) / 448).clamp_min(1e-12)
     want = (y.float() / scale).clamp(-448, 448).to(torch.float8_e4m3fn)
     assert torch.equal(y8.cpu().view(torch.uint8), want.view(torch.uint8))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_forward_of_items_of_one_to_three_ragged_kv_tiles(D):
+    """The loader asks for all tiles of an item of one or two KV tiles before it zeroes the ragged ones: every combination
+    of Q and KV lengths around one and two tiles, against fp64 within the bf16 bound of the kernels."""
+    import ads_model_kernel_library_b200.gdpa as G
+
+    g = torch.Generator().manual_seed(D)
+    edges = [1, 127, 128, 129, 255, 256, 257, 300]
+    lq, lk = [a for a in edges for _ in edges], [b for _ in edges for b in edges]
+    qo, ko = (torch.tensor(np.concatenate([[0], np.cumsum(n)])) for n in (lq, lk))
+    q = torch.randn(int(qo[-1]), 2, D, generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(int(ko[-1]), 2, D, generator=g).to(torch.bfloat16) for _ in range(2))
+    o = G.generalized_dot_product_attention(q.cuda(), k.cuda(), v.cuda(), qo.cuda(), ko.cuda(), 300, 300, qk_scale=1 / 64,
+                                            activation="gelu_approx")
+    torch.cuda.synchronize()
+    assert G.kernel_status() == 0
+    for b in range(len(lq)):
+        qb, (kb, vb) = q[qo[b]:qo[b + 1]].double(), (t[ko[b]:ko[b + 1]].double() for t in (k, v))
+        p = torch.nn.functional.gelu(torch.einsum("qhd,khd->hqk", qb, kb), approximate="tanh") / 64
+        assert_close(o[qo[b]:qo[b + 1]], torch.einsum("hqk,khd->qhd", p, vb), f"O[{lq[b]}, {lk[b]}]")
