@@ -229,3 +229,24 @@ def test_forward_of_items_of_one_to_three_ragged_kv_tiles(D):
         qb, (kb, vb) = q[qo[b]:qo[b + 1]].double(), (t[ko[b]:ko[b + 1]].double() for t in (k, v))
         p = torch.nn.functional.gelu(torch.einsum("qhd,khd->hqk", qb, kb), approximate="tanh") / 64
         assert_close(o[qo[b]:qo[b + 1]], torch.einsum("hqk,khd->qhd", p, vb), f"O[{lq[b]}, {lk[b]}]")
+
+
+@pytest.mark.parametrize("scale,value", [("0x1.2da85cp-1", 0.0), ("0x1.2da864p-1", 0.0), ("0x1.2da850p-1", 2.0 ** -9)])
+def test_fp8_softmax_rounds_the_exponent_before_the_factor_of_p(G, scale, value):
+    """P is stored as e4m3(2^7 exp2(x)), x = c S - m rounded to fp32.  The midpoint between 0 and the smallest e4m3, 2^-10,
+    is x = -17.  One key has S = 0 (m = 0, P = 2^7, its V row is 0), 127 have S = -20 and V = 1, so a row is
+    127 e4m3(2^7 exp2(x)) over the row sum.  With the first scale c S is 0.75 * 2^-20 above -17, which fp32 rounds to -17
+    (spacing 2^-19) and the conversion to 0; as a term of the exponent 2^7 would move the sum to -10, where the spacing is
+    2^-20, and P to 2^-9.  The second scale gives c S below -17, the third 5.4 * 2^-19 above."""
+    D = 128
+    q, k, v = (torch.zeros(128, 1, D) for _ in range(3))
+    q[:, 0, 0] = 1.0
+    k[1:, 0, 0] = -20.0
+    v[1:] = 1.0
+    off, blocks, one = torch.tensor([0, 128]).cuda(), torch.tensor([0, 1]).cuda(), torch.ones(1, 1).cuda()
+    o = G.generalized_dot_product_attention_fp8(*(t.to(torch.float8_e4m3fn).cuda() for t in (q, k, v)), one, one, one, blocks, blocks,
+                                                off, off, 128, 128, qk_scale=float.fromhex(scale))
+    torch.cuda.synchronize()
+    assert G.kernel_status() == 0
+    want = torch.tensor(127 * value / 128 / (1 + 127 * 2.0 ** -17)).to(torch.bfloat16)
+    assert torch.equal(o.cpu(), want.expand(o.shape))
