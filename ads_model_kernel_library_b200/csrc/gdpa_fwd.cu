@@ -493,9 +493,11 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         const float *k_scale = nullptr, *v_scale = nullptr;
         if constexpr (FP8) {
           sq = a.q_scales[static_cast<long long>(w.q_scale0 + s) * a.heads + w.h];
-          const long long at = static_cast<long long>(w.kv_scale0 + j0) * a.kv_heads + w.h / a.kv_group;
-          k_scale = a.k_scales + at, v_scale = a.v_scales + at;
-          sk_next = *k_scale, sv_next = *v_scale;
+          if (nkv > 0) {  // the row of an empty KV sequence at the end of the batch is past the end of the scales
+            const long long at = static_cast<long long>(w.kv_scale0 + j0) * a.kv_heads + w.h / a.kv_group;
+            k_scale = a.k_scales + at, v_scale = a.v_scales + at;
+            sk_next = *k_scale, sv_next = *v_scale;
+          }
         }
         for (int j = 0; j < nkv; ++j) {
           // columns [clo, chi) of this warp's 64 take part: inside the KV length and inside the band

@@ -250,3 +250,23 @@ def test_fp8_softmax_rounds_the_exponent_before_the_factor_of_p(G, scale, value)
     assert G.kernel_status() == 0
     want = torch.tensor(127 * value / 128 / (1 + 127 * 2.0 ** -17)).to(torch.bfloat16)
     assert torch.equal(o.cpu(), want.expand(o.shape))
+
+
+@pytest.mark.parametrize("act", ["softmax", "gelu_approx"])
+def test_fp8_forward_with_empty_kv_sequences_and_scales_of_exactly_the_blocks(G, act):
+    """A sequence without keys has no row in the scales: behind the last block there is nothing to read.  Its output rows
+    are zero; the other rows are those of the same call with the rows that the quantiser allocates behind the blocks."""
+    lq, lk = [130, 0, 300, 7, 40], [0, 64, 300, 0, 0]
+    g = torch.Generator().manual_seed(3)
+    qo, ko = (torch.tensor(np.concatenate([[0], np.cumsum(n)])).cuda() for n in (lq, lk))
+    q, k, v = (torch.randn(n, 2, 128, generator=g).to(torch.bfloat16).cuda() for n in (sum(lq), sum(lk), sum(lk)))
+    (q8, sq, qb), (k8, sk, kb), (v8, sv, _) = (G.quantize_fp8_blockwise(t, o) for t, o in ((q, qo), (k, ko), (v, ko)))
+    out = []
+    for rows in (len(sk), int(kb[-1])):
+        out.append(G.generalized_dot_product_attention_fp8(q8, k8, v8, sq, sk[:rows].clone(), sv[:rows].clone(), qb, kb, qo, ko, 300, 300,
+                                                           qk_scale=0.1, activation=act))
+        torch.cuda.synchronize()
+        assert G.kernel_status() == 0
+    assert torch.equal(out[0], out[1])
+    empty = torch.cat([out[1][:130], out[1][430:]])
+    assert bool((empty == 0).all()) and bool(out[1][130:430].isfinite().all()) and bool((out[1][130:430] != 0).any())
