@@ -165,7 +165,7 @@ gdpa_bwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
-  const int n_items = a.sched[0];
+  const int n_items = schedule_items(a.sched, a.sched[1] == kSchedBwd, a.status);
   const SeqLimits lim = {a.total_q, a.total_kv, 0};
 #ifdef GDPA_ENABLE_TRACE
   // every CTA's start and end time (ns) in the last 512 slots of the trace buffer

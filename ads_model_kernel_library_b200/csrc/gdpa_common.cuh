@@ -13,6 +13,15 @@ constexpr int kSchedHeaderInts = 4; // schedule buffer: int32 header {count, mod
 // row of the run this item takes, row past its last}
 constexpr int kSchedFwd = 0, kSchedBwd = 1, kSchedFwdShared = 2;
 
+// Number of items of a schedule, asked for by whole warps: none, and a status code, if it is of a kind (not `usable`) that the kernel
+// cannot walk -- another mode's items name rows and blocks that this kernel would turn into addresses.
+__device__ __forceinline__ int schedule_items(const int* sched, bool usable, int* status) {
+  if (usable) return sched[0];
+  if (status != nullptr && (threadIdx.x & 31) == 0 && *reinterpret_cast<volatile int*>(status) == 0)
+    *reinterpret_cast<volatile int*>(status) = (sched[1] << 8) | ST_SCHEDULE;
+  return 0;
+}
+
 // Activation classes the kernels are specialised on (several reference names share one class).
 enum ActClass : int {
   ACT_RAW = 0,

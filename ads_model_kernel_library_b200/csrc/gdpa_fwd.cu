@@ -167,7 +167,6 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
-  const int n_items = a.sched[0];
   const SeqLimits lim = {a.total_q, a.total_kv, a.kv_batch};
 
   // The loader warp walks the list, reads an item and its sequence's offsets (two dependent trips to memory, with FP8
@@ -242,25 +241,29 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         if (lane == 0) mbar_arrive(bar_base + 8u * full_bar);
         return true;
       };
-      WorkWalker walker(n_items);
-      const bool shared_runs = a.sched[1] == kSchedFwdShared;
+      // runs of sequences have no block scales of their own (FP8), no positions in a sequence (a window), and need the
+      // KV sequence's index
+      const bool shared_runs = !FP8 && a.sched[1] == kSchedFwdShared && a.window < 0 && a.kv_index != nullptr;
+      WorkWalker walker(schedule_items(a.sched, shared_runs || a.sched[1] == kSchedFwd, a.status));
       // producer side of the work ring: the slot must have been read by every consumer of its previous use
       auto next_item = [&](Item& it) -> bool {
         const uint32_t slot = work_pos % kWorkSlots, parity = (work_pos / kWorkSlots) & 1u;
         it = Item{-1, 0, 0, 0, 0, 0, 0, 0, 0, 0};
         int i;
         if (walker.next(i)) {
-          const Work w = load_work(a.sched, i, a.q_off, a.kv_off, a.off64, a.max_q, a.max_kv, lim, a.kv_index);
-          it.h = w.h, it.q0 = w.blk * kFwdQBlock;
+          Work w = load_work(a.sched, i, a.q_off, a.kv_off, a.off64, a.max_q, a.max_kv, lim, a.kv_index);
+          it.h = w.h;
           it.q_start = static_cast<int>(w.q_start), it.kv_start = static_cast<int>(w.kv_start);
-          it.lq = w.lq, it.lkv = w.lkv;
-          fwd_kv_range(w, a.window, it.j0, it.nkv);
           if (shared_runs) {
             // rows of a run of sequences instead of a block of one, still clamped to the tensor
             const int4 run = reinterpret_cast<const int4*>(a.sched + kSchedHeaderInts)[i];
+            w.blk = 0;
+            w.lq = static_cast<int>(min(static_cast<long long>(run.w), a.total_q - w.q_start));
             it.q0 = run.z;
-            it.lq = static_cast<int>(min(static_cast<long long>(run.w), a.total_q - w.q_start));
           }
+          it.q0 += w.blk * kFwdQBlock;
+          it.lq = w.lq, it.lkv = w.lkv;
+          fwd_kv_range(w, a.window, it.j0, it.nkv);
           if constexpr (FP8) {
             it.q_scale0 = static_cast<int>(load_offset(a.q_blk_off, w.b, a.off64)) + w.blk * 2;
             it.kv_scale0 = static_cast<int>(load_offset(a.kv_blk_off, w.kb, a.off64));

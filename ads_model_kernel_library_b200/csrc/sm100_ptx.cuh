@@ -11,7 +11,7 @@
 namespace gdpa {
 
 // ----------------------------------------------------------------------------------------------
-// Status codes written to the caller's status word when a bounded wait runs out.
+// Status codes written to the caller's status word when a bounded wait runs out (or a schedule is refused).
 // The low byte says which role gave up, the rest which barrier.
 // ----------------------------------------------------------------------------------------------
 enum : int {
@@ -22,6 +22,7 @@ enum : int {
   ST_ROLE_EPI = 4,
   ST_ROLE_RED = 5,
   ST_ROLE_FIX = 6,
+  ST_SCHEDULE = 7,  // not a wait: the schedule is of a kind the kernel cannot walk; the rest is the mode it found
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

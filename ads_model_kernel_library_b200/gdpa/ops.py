@@ -82,6 +82,9 @@ def _status_word(device: torch.device) -> torch.Tensor:
 
 
 def _describe_status(code: int) -> str:
+    if code & 0xff == 7:
+        return (f"a kernel was given a schedule of mode {code >> 8}, which it cannot walk (status 0x{code:x}); "
+                "it has written no results")
     return (f"a kernel wait ran out (status 0x{code:x}: barrier {code >> 8}, role {_ROLE_NAMES.get(code & 0xff, code & 0xff)}); "
             "results of the calls since the last check on this device are incomplete")
 

@@ -30,6 +30,8 @@
  *  - Every in-kernel wait is bounded.  A wait that runs out writes a non-zero code to
  *    `status` (if given), the kernel frees its tensor memory and returns; the context stays
  *    usable.
+ *  - A kernel that is given a schedule of a mode it cannot walk (see GDPA_SCHED_*) writes the code
+ *    mode << 8 | 7 to `status` (if given) and no results.
  *  - Offsets are trusted to be monotone prefix sums inside the tensors.  The kernels clamp every sequence range
  *    they read from an offset array to [0, total_q] / [0, total_kv], so a malformed array gives unspecified values
  *    for the sequences concerned but no access outside the tensors; checking the arrays is the host's business.
@@ -93,7 +95,7 @@ enum {
   /* Forward with kv_seq_index and no window: neighbouring Q sequences that read the same KV sequence are taken
    * together, one work item per (run of sequences, head, 256- or 128-row Q block).  For gdpa_fwd only (not for
    * gdpa_fwd_fp8, whose scales are per sequence, and not for a call with a window, which counts positions in the
-   * sequence). */
+   * sequence: there the kernel refuses it). */
   GDPA_SCHED_FWD_SHARED_KV = 2
 };
 
@@ -157,10 +159,10 @@ typedef struct GdpaFwdParams {
   int32_t max_seq_len_kv;
   int32_t activation;         /* GDPA_ACT_* */
   float qk_scale;             /* multiplies act(S); for softmax multiplies S before exp */
-  const void* schedule;       /* from gdpa_build_schedule(GDPA_SCHED_FWD) */
+  const void* schedule;       /* from gdpa_build_schedule(GDPA_SCHED_FWD or GDPA_SCHED_FWD_SHARED_KV) */
   int32_t* status;            /* optional int32 in device memory, or in pinned host memory mapped into the device's
                                  address space (the host can then poll it without a synchronisation); written
-                                 non-zero if a wait ran out */
+                                 non-zero if a wait ran out or the schedule was refused */
   /* FP8 path only (gdpa_fwd_fp8): one fp32 scale per (sequence-local 128-token block, head),
    * laid out [number of blocks over the batch, heads]; block b of sequence s sits at row
    * block_offsets[s] + b where block_offsets is the exclusive prefix sum of ceil(len / 128). */

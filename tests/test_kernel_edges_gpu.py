@@ -270,3 +270,39 @@ def test_fp8_forward_with_empty_kv_sequences_and_scales_of_exactly_the_blocks(G,
     assert torch.equal(out[0], out[1])
     empty = torch.cat([out[1][:130], out[1][430:]])
     assert bool((empty == 0).all()) and bool(out[1][130:430].isfinite().all()) and bool((out[1][130:430] != 0).any())
+
+
+@pytest.mark.parametrize("call,mode", [("fp8", 2), ("fp8", 1), ("window", 2), ("no index", 2), ("no index", 1), ("backward", 0),
+                                       ("backward", 2)])
+def test_a_kernel_refuses_a_schedule_it_cannot_walk(G, monkeypatch, call, mode):
+    """Items of another mode name other rows and blocks: the kernel walks none of them, writes the mode it found to the
+    status word, and the next call raises it."""
+    from ads_model_kernel_library_b200.gdpa import _cabi, ops
+
+    D, lens = 128, [300, 5, 700]
+    off = torch.tensor(np.concatenate([[0], np.cumsum(lens)])).cuda()
+    index = torch.arange(len(lens)).cuda()
+    g = torch.Generator().manual_seed(1)
+    q, k, v = (torch.randn(sum(lens), 2, D, generator=g).to(torch.bfloat16).cuda().requires_grad_(call == "backward") for _ in range(3))
+    build = ops._build_schedule
+
+    def other_mode(wanted, qo, ko, batch, heads, rows, max_q, max_kv, kv_index=None, start_end=False):
+        wrong = (wanted == _cabi.GDPA_SCHED_BWD) if call == "backward" else True
+        return build(mode if wrong else wanted, qo, ko, batch, heads, rows, max_q, max_kv, index if wrong and mode == 2 else kv_index)
+
+    monkeypatch.setattr(ops, "_build_schedule", other_mode)
+    if call == "fp8":
+        (q8, sq, b), (k8, sk, _), (v8, sv, _) = (G.quantize_fp8_blockwise(t, off) for t in (q, k, v))
+        G.generalized_dot_product_attention_fp8(q8, k8, v8, sq, sk, sv, b, b, off, off, 700, 700)
+    elif call == "window":
+        G.generalized_dot_product_attention(q, k, v, off, off, 700, 700, ad_to_request_offset=index, window_size=64)
+    else:
+        o = G.generalized_dot_product_attention(q, k, v, off, off, 700, 700, activation="relu")
+        if call == "backward":
+            o.sum().backward()
+    torch.cuda.synchronize()
+    monkeypatch.undo()
+    with pytest.raises(RuntimeError, match=f"schedule of mode {mode}"):
+        G.generalized_dot_product_attention(q, k, v, off, off, 700, 700, activation="relu")
+    G.generalized_dot_product_attention(q, k, v, off, off, 700, 700, activation="relu")
+    assert G.kernel_status() == 0
