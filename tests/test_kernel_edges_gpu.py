@@ -159,10 +159,8 @@ def test_shared_kv_runs_cover_every_row_once(requests, per, rows, heads):
 @pytest.mark.parametrize("D,act", [(64, "silu"), (128, "gelu_approx"), (128, "softmax")])
 @pytest.mark.parametrize("per,rows", [(7, 20), (150, 90)])
 def test_shared_kv_runs_give_what_single_sequences_give(G, D, act, per, rows):
-    """The same call with a band that reaches every pair is scheduled sequence by sequence.  Same products; the fp32 sums
-    may be split over the two accumulators differently (some 1e-7 of the sum of at most 700 terms of a few units: 1e-3),
-    and one that lies near a rounding boundary then differs by an ulp of bf16, 2^-7.  (Softmax: when a row's running
-    maximum moves depends on the rows beside it, so its P is rounded to bf16 from another base, a few such ulps.)"""
+    """The same call with a band that reaches every pair is scheduled sequence by sequence.  A row's products, and the order
+    of its fp32 sums over the KV tiles, are the same in both: so are the results."""
     g = torch.Generator().manual_seed(per)
     rng = np.random.default_rng(per)
     requests, H = 3, 2
@@ -175,7 +173,31 @@ def test_shared_kv_runs_give_what_single_sequences_give(G, D, act, per, rows):
                                                window_size=w) for w in (None, 1 << 20)]
     torch.cuda.synchronize()
     assert G.kernel_status() == 0
-    assert_close(out[0], out[1], "runs", atol=1e-2 if act == "softmax" else 1e-3, rtol=1e-2 if act == "softmax" else 2.0 ** -7)
+    assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("act", ["softmax", "silu", "relu"])
+def test_shared_kv_result_does_not_depend_on_the_sequences_beside_it(G, act):
+    """Candidates of one request, in one Q tile, with keys that grow: the scores of the second stay within a few units, so that
+    alone its softmax keeps the maximum of the first tile, while those of the others (with a factor of 32) move theirs from
+    tile to tile.  The rows of the second are the same bits whatever the others hold, infinities and NaN included."""
+    g = torch.Generator().manual_seed(5)
+    D, lq, kv = 128, [20, 40, 30], 900
+    qo, ko = (torch.tensor(np.concatenate([[0], np.cumsum(n)])).cuda() for n in (lq, [kv]))
+    q = torch.randn(sum(lq), 2, D, generator=g).to(torch.bfloat16).cuda()
+    k, v = (torch.randn(kv, 2, D, generator=g).cuda() for _ in range(2))
+    k, v = (k * torch.linspace(0.2, 3.0, kv).cuda().view(-1, 1, 1)).to(torch.bfloat16), v.to(torch.bfloat16)
+    rows = []
+    for factor in (1.0, 0.0, 32.0, float("inf")):
+        x = q.clone()
+        x[:20] *= factor
+        x[60:] *= -factor
+        o = G.generalized_dot_product_attention(x, k, v, qo, ko, 40, kv, ad_to_request_offset=torch.zeros(3, dtype=torch.int64).cuda(),
+                                                qk_scale=0.02, activation=act)
+        torch.cuda.synchronize()
+        assert G.kernel_status() == 0
+        rows.append(o[20:60])
+    assert rows[0].isfinite().all() and all(torch.equal(rows[0], r) for r in rows[1:])
 
 
 @pytest.mark.parametrize("D", [64, 128])
