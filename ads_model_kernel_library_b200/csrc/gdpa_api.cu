@@ -482,6 +482,7 @@ int gdpa_bwd(const GdpaBwdParams* p, gdpa_stream_t stream) {
   if (p->k == nullptr || p->v == nullptr || p->dk == nullptr || p->dv == nullptr) return GDPA_ERR_BAD_ARG;
   if (((reinterpret_cast<uintptr_t>(p->dk) | reinterpret_cast<uintptr_t>(p->dv) | reinterpret_cast<uintptr_t>(p->dq)) & 15u) != 0)
     return GDPA_ERR_MISALIGNED;
+  if (act == ACT_SOFTMAX && (reinterpret_cast<uintptr_t>(p->o) & 3u) != 0) return GDPA_ERR_MISALIGNED;  // read by words at least
   const bool pairs = (p->offsets_are_int64 & GDPA_OFFSETS_PAIRS) != 0;
   if (pairs && p->dkv_accum == nullptr) return GDPA_ERR_BAD_ARG;
   if (pairs && (reinterpret_cast<uintptr_t>(p->dkv_accum) & 15u) != 0) return GDPA_ERR_MISALIGNED;

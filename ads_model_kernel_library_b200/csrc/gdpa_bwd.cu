@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(256) gdpa_dq_convert_kernel(const float4* __re
 constexpr int kDpsumThreads = 256;
 template <int D>
 constexpr int kDpsumTokens = 4 * kDpsumThreads / (D / 8);
-template <int D, bool O16>  // O16: `o` is 16-byte aligned (dO is, its tensor map asks for it); else it is read by words
+template <int D, bool O16>  // O16: `o` is 16-byte aligned (dO is, its tensor map asks for it); else by words, 4-byte aligned
 __global__ void __launch_bounds__(kDpsumThreads) gdpa_dpsum_kernel(const __nv_bfloat16* __restrict__ d_o,
                                                                    const __nv_bfloat16* __restrict__ o,
                                                                    float* __restrict__ dpsum, long long total_q, int heads) {

@@ -398,7 +398,7 @@ typedef struct GdpaBwdParams {
   void* timing_stop_event;
   /* GDPA_ACT_SOFTMAX only (the softmax backward, which the reference leaves unimplemented:
    * gdpa/src/flash_bwd_sm100.py:2038-2058 keeps the dPsum term commented out): the forward output O
-   * [total_q, heads, head_dim] bf16, the forward's lse [heads, total_q] fp32, and a scratch buffer of
+   * [total_q, heads, head_dim] bf16, 4-byte aligned (16-byte aligned is faster), the forward's lse [heads, total_q] fp32, and a scratch buffer of
    * total_q * heads floats that receives dPsum = rowsum(dO * O). */
   const void* o;
   const float* lse;

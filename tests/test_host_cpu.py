@@ -65,6 +65,17 @@ def test_argument_checks_before_any_cuda_call(cabi):
     assert b"head_dim" in cabi.lib.gdpa_strerror(2)
 
 
+def test_softmax_backward_refuses_an_output_that_words_cannot_be_read_from(cabi):
+    p = cabi.GdpaBwdParams()
+    p.struct_size = C.sizeof(cabi.GdpaBwdParams)
+    p.heads, p.head_dim, p.batch, p.total_q, p.total_kv = 2, 128, 1, 1, 1
+    for name in ("q", "k", "v", "d_o", "dq", "dk", "dv", "dq_accum", "q_offsets", "kv_offsets", "schedule", "lse", "dpsum"):
+        setattr(p, name, 16)
+    p.activation = 100
+    for p.o in (17, 18, 19, 30):
+        assert cabi.lib.gdpa_bwd(C.byref(p), None) == 5
+
+
 def test_mxfp8_entry_points_check_arguments_before_any_cuda_call(cabi):
     for fn in (cabi.lib.gdpa_quantize_mxfp8, cabi.lib.gdpa_dequantize_mxfp8):
         p = cabi.GdpaMxParams()
