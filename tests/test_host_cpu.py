@@ -219,3 +219,16 @@ def test_clock_sampler_keeps_the_samples_of_the_timed_region_only():
     s2.proc = Proc()
     s2.lines = [idle] * 2
     assert s2.stop(s2.mark(0.0))["samples"] == 1
+
+
+def test_launching_helpers_refuse_a_tensor_that_is_not_on_a_gpu():
+    """A host pointer must not reach a kernel: norm_rows_backward has no check of its own before the device is entered."""
+    from ads_model_kernel_library_b200.gdpa import ops
+    from ads_model_kernel_library_b200.gdpa.megakernel import norm_rows_backward
+
+    rows = torch.zeros(2, 8, dtype=torch.bfloat16)
+    for t in (rows, rows.to("meta")):
+        with pytest.raises(ValueError, match="cuda device"):
+            ops._on_device(t)
+    with pytest.raises(ValueError, match="cuda device"):
+        norm_rows_backward(2, rows, rows)
