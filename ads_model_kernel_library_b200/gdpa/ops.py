@@ -61,6 +61,12 @@ def _device_key(device: torch.device) -> int:
     return device.index if device.index is not None else torch.cuda.current_device()
 
 
+# Private names of torch, for the host time they save; a torch without them gets its public functions.
+_device_guard = getattr(torch.cuda, "_DeviceGuard", torch.cuda.device)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+
+
 def _on_device(t: torch.Tensor):
     """The device of a CUDA tensor as the current one (``torch.cuda.device`` without its look at what else it may be given).
 
@@ -68,7 +74,7 @@ def _on_device(t: torch.Tensor):
     read without a tensor operation and one look at each tensor's strides 387 us became 279 us."""
     if not t.is_cuda:
         raise ValueError(f"Expected a cuda device, but got: {t.device}")
-    return torch.cuda._DeviceGuard(t.get_device())
+    return _device_guard(t.get_device())
 
 
 def _status_word(device: torch.device) -> torch.Tensor:
@@ -154,8 +160,10 @@ def _maybe_validate(qo, ko, total_q: int, total_kv: int, start_end: bool = False
 
 
 def _stream_ptr() -> int:
-    """The current stream of the current device as an integer (no ``torch.cuda.Stream`` object is made for it)."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    """The current stream of the current device as an integer (without a ``torch.cuda.Stream`` object made for it)."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def _check_inputs(q, k, v, qo, ko, dtype, shared_kv: bool = False, start_end: bool = False) -> Tuple[int, int, int]:

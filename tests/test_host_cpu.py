@@ -232,3 +232,21 @@ def test_launching_helpers_refuse_a_tensor_that_is_not_on_a_gpu():
             ops._on_device(t)
     with pytest.raises(ValueError, match="cuda device"):
         norm_rows_backward(2, rows, rows)
+
+
+def test_module_loads_and_finds_the_stream_without_torch_private_names():
+    """A torch that has renamed what the host path takes from its private parts: in a process of its own, with the names
+    deleted before the package is imported."""
+    import subprocess
+    import sys
+
+    code = """
+import types, torch
+for owner, name in ((torch.cuda, "_DeviceGuard"), (torch._C, "_cuda_getCurrentRawStream"), (torch._C, "_cuda_getDevice")):
+    if hasattr(owner, name):
+        delattr(owner, name)
+from ads_model_kernel_library_b200.gdpa import ops
+torch.cuda.current_stream = lambda: types.SimpleNamespace(cuda_stream=77)
+assert ops._stream_ptr() == 77 and ops._device_guard is torch.cuda.device
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT, timeout=300)
