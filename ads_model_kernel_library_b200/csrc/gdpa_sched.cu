@@ -94,14 +94,19 @@ __device__ __forceinline__ void run_geometry(const SchedArgs& a, int b0, int n, 
 
 // Latency-bound: one block, a few thousand items, and the forward or backward kernel waits for it.  What it costs is the
 // chain of dependent steps, so: only the bins that a sequence of the given maximum length can have are cleared and
-// scanned (17 of 4096 for 2048 tokens), the scan gives each thread its own run of neighbouring bins (a warp reads
-// consecutive words, no bank conflicts) instead of one warp walking all of them, and the items of a chunk of 1024
-// sequences are written by all warps together, 32 consecutive items (512 bytes) per store, instead of each thread
-// writing the items of one sequence one after another (13 -> 4 us for 8 sequences, 26 -> 15 us for 1024).
+// scanned (17 of 4096 for 2048 tokens), and the scan gives each thread its own run of neighbouring bins (a warp reads
+// consecutive words, no bank conflicts) instead of one warp walking all of them.  With many sequences it is the number of
+// instructions: without runs no warp waits for another between two sequences, and a warp writes the items of its sequences
+//  - each lane its own sequence's, if none has more than four (100 000 sequences of one head: 168 us);
+//  - one sequence after another, 32 items (512 bytes) a store, if they have 64 and more on average;
+//  - otherwise 32 items at a time across its sequences (100 000 sequences of 8 heads: 458 us, 642 us with a lane for each
+//    sequence, 1216 us with a warp for each).
+// Launch and kernel of a build, back to back: 8 sequences 15 -> 10 us; 1152 of up to 100 tokens and 8 heads 21 -> 11 us, of
+// up to 2000 tokens 42 -> 21 us (from a warp that walks all bins and a lane for each sequence).
 __global__ void __launch_bounds__(kSchedThreads, 1) gdpa_build_schedule_kernel(const SchedArgs a) {
   __shared__ int hist[kBins];
   __shared__ int warp_sum[kSchedThreads / 32];
-  __shared__ int4 seq[kSchedThreads];  // of the sequences of one chunk: first slot, blocks, weight, rows (of a run)
+  __shared__ int4 seq[kSchedThreads + kSchedThreads / 32];  // first slot, blocks, weight, rows of a run; a gap after every 32
   __shared__ int first_head[kSchedThreads / 32];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const bool shared = a.mode == kSchedFwdShared;
@@ -116,12 +121,18 @@ __global__ void __launch_bounds__(kSchedThreads, 1) gdpa_build_schedule_kernel(c
   if (shared && a.batch > 0 &&
       (load_offset(a.q_off, a.batch, a.off64) - load_offset(a.q_off, 0, a.off64)) / kFwdQBlock * a.heads < kSms)
     piece = kTile;
+  // Chunks of up to 1024 sequences, a sequence per thread, dealt out evenly to the warps (runs: in the order of the threads).
   int nblk = 0, w = 0, rows = 0;  // of this thread's sequence of the last chunk: the only one unless the batch is large
+  auto geometry = [&](int b0, int n, int each) {
+    const int mine = warp * each + lane;
+    if (shared) run_geometry(a, b0, n, piece, first_head, nblk, w, rows);
+    else if (lane < each && mine < n) seq_geometry(a, b0 + mine, nblk, w);
+    else nblk = 0;
+  };
   for (int b0 = 0; b0 < a.batch; b0 += kSchedThreads) {
     const int n = min(kSchedThreads, a.batch - b0);
-    if (shared) run_geometry(a, b0, n, piece, first_head, nblk, w, rows);
-    else if (t < n) seq_geometry(a, b0 + t, nblk, w);
-    if (t < n && nblk > 0) atomicAdd(&hist[w], nblk * a.heads);
+    geometry(b0, n, shared ? 32 : (n + 31) / 32);
+    if (nblk > 0) atomicAdd(&hist[w], nblk * a.heads);
   }
   __syncthreads();
   // Exclusive prefix over bins from the heaviest down: hist[w] becomes the first slot of weight w.  Thread t owns the
@@ -156,28 +167,72 @@ __global__ void __launch_bounds__(kSchedThreads, 1) gdpa_build_schedule_kernel(c
   }
   __syncthreads();
   int4* items = reinterpret_cast<int4*>(a.sched + kSchedHeaderInts);
+  auto put = [&](long long slot, int b, int h, int blk, int last) {  // last: the weight, or the rows of a run
+    if (slot < cap)
+      items[slot] = shared ? make_int4(b, h, blk * piece, min(last, (blk + 1) * piece)) : make_int4(b, h, blk, last);
+  };
+  // k / blocks: (k + 0.5) / blocks is at least 0.5 / blocks away from a whole number, further than it is rounded for k < 2^21
+  auto head_of = [&](int k, int blocks, float inv) {
+    return k < (1 << 21) ? static_cast<int>((static_cast<float>(k) + 0.5f) * inv) : k / blocks;
+  };
+  // The items of a warp's sequences: lane `src` holds sequence first_b + src * step_b, its first slot, blocks, weight and rows.
+  auto put_items = [&](const int4& sq, int first_b, int step_b) {
+    const int count = sq.y * a.heads, my_last = shared ? sq.w : sq.z;
+    if (!__any_sync(0xffffffffu, count > 4)) {
+      for (int k = 0, h = 0, blk = 0; k < count; ++k) {
+        put(static_cast<long long>(sq.x) + k, first_b + lane * step_b, h, blk, my_last);
+        if (++blk == sq.y) blk = 0, ++h;
+      }
+      return;
+    }
+    int end = count;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, end, d);
+      if (lane >= d) end += n;
+    }
+    const int begin = end - count, all = __shfl_sync(0xffffffffu, end, 31);
+    const float my_inv = 1.f / static_cast<float>(sq.y);
+    unsigned left = __ballot_sync(0xffffffffu, count > 0);
+    if (all >= 64 * __popc(left)) {
+      for (; left != 0u; left &= left - 1u) {
+        const int src = __ffs(left) - 1;
+        const int slot = __shfl_sync(0xffffffffu, sq.x, src), nb = __shfl_sync(0xffffffffu, sq.y, src);
+        const int last = __shfl_sync(0xffffffffu, my_last, src), n = __shfl_sync(0xffffffffu, count, src);
+        const float inv = __shfl_sync(0xffffffffu, my_inv, src);
+        for (int k = lane; k < n; k += 32) {
+          const int h = head_of(k, nb, inv);
+          put(static_cast<long long>(slot) + k, first_b + src * step_b, h, k - h * nb, last);
+        }
+      }
+      return;
+    }
+    for (int i0 = 0; i0 < all; i0 += 32) {
+      const int i = i0 + lane;
+      int src = 0;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1)
+        if (__shfl_sync(0xffffffffu, end, src + d - 1) <= i) src += d;
+      const int k = i - __shfl_sync(0xffffffffu, begin, src), slot = __shfl_sync(0xffffffffu, sq.x, src);
+      const int nb = __shfl_sync(0xffffffffu, sq.y, src), last = __shfl_sync(0xffffffffu, my_last, src);
+      const int h = head_of(k, nb, __shfl_sync(0xffffffffu, my_inv, src));
+      if (i < all) put(static_cast<long long>(slot) + k, first_b + src * step_b, h, k - h * nb, last);
+    }
+  };
+  const bool one_chunk = a.batch <= kSchedThreads;
   for (int b0 = 0; b0 < a.batch; b0 += kSchedThreads) {
     const int n = min(kSchedThreads, a.batch - b0);
-    if (a.batch > kSchedThreads) {
-      if (shared) run_geometry(a, b0, n, piece, first_head, nblk, w, rows);
-      else if (t < n) seq_geometry(a, b0 + t, nblk, w);
+    const int each = shared ? 32 : (n + 31) / 32;
+    if (!one_chunk) geometry(b0, n, each);
+    const int count = nblk * a.heads;
+    const int4 sq = make_int4(count > 0 ? atomicAdd(&hist[w], count) : 0, nblk, w, rows);
+    if (shared && one_chunk) {  // the few first sequences of runs: dealt out to the warps one by one
+      seq[t + warp] = sq;
+      __syncthreads();
+      put_items(seq[lane * 33 + warp], warp, 32);
+    } else {
+      put_items(sq, b0 + warp * each, 1);
     }
-    if (t < n) {
-      const int count = nblk * a.heads;
-      seq[t] = make_int4(count > 0 ? atomicAdd(&hist[w], count) : 0, nblk, w, rows);
-    }
-    __syncthreads();
-    for (int i = warp; i < n; i += kSchedThreads / 32) {
-      const int4 sq = seq[i];
-      const int count = sq.y * a.heads;
-      for (int k = lane; k < count; k += 32) {
-        const long long slot = static_cast<long long>(sq.x) + k;
-        const int h = k / sq.y, blk = k - h * sq.y;
-        if (slot < cap)
-          items[slot] = shared ? make_int4(b0 + i, h, blk * piece, min(sq.w, (blk + 1) * piece)) : make_int4(b0 + i, h, blk, sq.z);
-      }
-    }
-    __syncthreads();
   }
   if (t == 0) {
     a.sched[0] = static_cast<int>(total < cap ? total : cap);

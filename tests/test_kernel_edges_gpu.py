@@ -60,14 +60,18 @@ def _schedule(qo, ko, mode, heads, max_q, max_kv, kv_index=None):
     return s[:4].tolist(), s[4:4 + 4 * int(s[0])].view(-1, 4)
 
 
+@pytest.mark.parametrize("heads,longest", [(3, 700), (1, 120), (7, 120), (5, 20000)])
 @pytest.mark.parametrize("batch", [1, 31, 1023, 1024, 1025, 2500])
 @pytest.mark.parametrize("mode", [0, 1])
-def test_schedule_lists_every_block_once_longest_first(mode, batch):
+def test_schedule_lists_every_block_once_longest_first(mode, batch, heads, longest):
+    """Some, at most four, seven and over 64 items a sequence."""
     rng = np.random.default_rng(batch)
-    lq, lk = rng.integers(0, 700, batch), rng.integers(0, 3000, batch)
-    lq[0] = lk[0] = 700
+    lq, lk = rng.integers(0, longest, batch), rng.integers(0, 4 * longest, batch)
+    lq[0] = lk[0] = longest
+    if longest == 20000:
+        lq[batch // 2:], lk[batch // 2:] = 15000, 8000
     qo, ko = (torch.tensor(np.concatenate([[0], np.cumsum(n)])).cuda() for n in (lq, lk))
-    heads, max_q, max_kv = 3, 600, 2500
+    max_q, max_kv = longest * 6 // 7, longest * 25 // 7
     header, items = _schedule(qo, ko, mode, heads, max_q, max_kv)
     tiles = lambda n, t: -(-n // t)  # noqa: E731
     cq, ck = np.minimum(lq, max_q), np.minimum(lk, max_kv)
