@@ -342,7 +342,9 @@ __global__ void __launch_bounds__(kNormThreads) gdpa_sum_rows_kernel(const NormB
   }
 }
 
-// Rows of more than kNormBwdMaxN values (no weight or bias gradients there): one warp per row, the row read twice.
+// The rows' gradients alone (no column sums, rows of any length): one warp per row, which reads the row twice, the second
+// time from L1 / L2.  HBM-bound like the kernel above, but with 60 (RMS norm) and 48 registers four and five blocks are
+// resident, so more rows are in flight, and a row need not fill the registers of whole warps.
 template <int MODE>
 __global__ void __launch_bounds__(kNormThreads) gdpa_norm_rows_bwd_wide_kernel(const NormBwdArgs a) {
   const int lane = threadIdx.x & 31;
@@ -356,44 +358,51 @@ __global__ void __launch_bounds__(kNormThreads) gdpa_norm_rows_bwd_wide_kernel(c
     uint4* dx = reinterpret_cast<uint4*>(a.dx + row * a.n);
     const float rstd = a.row_rstd[row];
     const float mean = MODE == 1 ? a.row_mean[row] : 0.f;
-    auto load = [&](int c, float (&gw)[8], float (&xh)[8]) {
-      unpack8(dy[c], gw);
+    // pass 1: the row sums
+    float s1 = 0.f, s2 = 0.f;
+    for (int c = lane; c < chunks; c += 32) {
+      float g[8], xv[8], w[8];
+      unpack8(dy[c], g);
       if (dy2 != nullptr) {
         float t[8];
         unpack8(dy2[c], t);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) gw[j] += t[j];
+        for (int j = 0; j < 8; ++j) g[j] += t[j];
       }
-      if (a.weight != nullptr) {
-        float w[8];
-        load8(a.weight + 8 * c, w);
+      unpack8(x[c], xv);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) gw[j] *= w[j];
-      }
-      unpack8(x[c], xh);
-      if (MODE == 1) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) xh[j] = (xh[j] - mean) * rstd;
-      }
-    };
-    float s1 = 0.f, s2 = 0.f;
-    for (int c = lane; c < chunks; c += 32) {
-      float gw[8], xh[8];
-      load(c, gw, xh);
+      for (int j = 0; j < 8; ++j) w[j] = 1.f;
+      if (a.weight != nullptr) load8(a.weight + 8 * c, w);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        s1 += gw[j];
-        s2 = fmaf(gw[j], xh[j], s2);
+        const float gw = g[j] * w[j];
+        const float xh = MODE == 1 ? (xv[j] - mean) * rstd : xv[j];
+        s1 += gw;
+        s2 = fmaf(gw, xh, s2);
       }
     }
     s1 = warp_sum(s1) * inv_n;
     s2 = warp_sum(s2) * inv_n;
+    // pass 2: dx
     for (int c = lane; c < chunks; c += 32) {
-      float gw[8], xh[8], o[8];
-      load(c, gw, xh);
+      float g[8], xv[8], w[8], o[8];
+      unpack8(dy[c], g);
+      if (dy2 != nullptr) {
+        float t[8];
+        unpack8(dy2[c], t);
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        o[j] = MODE == 0 ? rstd * (gw[j] - xh[j] * rstd * rstd * s2) : rstd * (gw[j] - s1 - xh[j] * s2);
+        for (int j = 0; j < 8; ++j) g[j] += t[j];
+      }
+      unpack8(x[c], xv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = 1.f;
+      if (a.weight != nullptr) load8(a.weight + 8 * c, w);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float gw = g[j] * w[j];
+        if (MODE == 0) o[j] = rstd * (gw - xv[j] * rstd * rstd * s2);
+        else o[j] = rstd * (gw - s1 - (xv[j] - mean) * rstd * s2);
+      }
       dx[c] = pack8(o);
     }
   }
@@ -403,12 +412,26 @@ template <int MODE>
 void launch_norm_bwd_mode(const NormBwdArgs& a, cudaStream_t stream) {
   // warps per row: the fewest that hold the row, 512 values each
   const int wpr = a.n <= 512 ? 1 : a.n <= 1024 ? 2 : a.n <= 2048 ? 4 : 8;
+  // Without column sums the register kernel is the faster one only where the row fills its lanes: by three quarters where no
+  // barrier is waited for (one warp) or the second reading would come from L2 (eight), and then for both norms; in between
+  // by more than 7/8 and for the RMS norm.  2^27 values, register kernel and the other one: RMS norm 64 values a row 825 and
+  // 695 us, 520: 284 and 221, 512: 168 and 195, 1024: 180 and 188, 3072: 205 and 254; layer norm 64: 1153 and 711, 1024: 227
+  // and 185, 2056: 342 and 209, 3584: 239 and 275.
+  const int held = 512 * wpr;
+  const bool sums = a.dweight != nullptr || (MODE == 1 && a.dbias != nullptr);
+  const bool filled = 4 * a.n >= 3 * held && (wpr == 1 || wpr == 8 || (MODE == 0 && 8 * a.n > 7 * held));
+  if (a.n > kNormBwdMaxN || (!sums && !filled)) {
+    // two rounds of the resident blocks; of the longer rows of the layer norm, which evict one another from L1, one per warp
+    const long long most = MODE == 0 ? 148 * 8 : a.n <= 1536 ? 148 * 10 : 1 << 30;
+    const long long blocks = (a.rows + kNormThreads / 32 - 1) / (kNormThreads / 32);
+    gdpa_norm_rows_bwd_wide_kernel<MODE><<<static_cast<unsigned>(blocks < most ? blocks : most), kNormThreads, 0, stream>>>(a);
+    return;
+  }
   const int groups = kNormThreads / 32 / wpr;
   const long long most = 148 * kNormBwdResident<MODE>;  // every block flushes its column sums once
   const long long blocks = (a.rows + groups - 1) / groups;
   const unsigned grid = static_cast<unsigned>(blocks < most ? blocks : most);
-  if (a.n > kNormBwdMaxN) gdpa_norm_rows_bwd_wide_kernel<MODE><<<grid * 2, kNormThreads, 0, stream>>>(a);
-  else if (wpr == 1) gdpa_norm_rows_bwd_kernel<MODE, 1><<<grid, kNormThreads, 0, stream>>>(a);
+  if (wpr == 1) gdpa_norm_rows_bwd_kernel<MODE, 1><<<grid, kNormThreads, 0, stream>>>(a);
   else if (wpr == 2) gdpa_norm_rows_bwd_kernel<MODE, 2><<<grid, kNormThreads, 0, stream>>>(a);
   else if (wpr == 4) gdpa_norm_rows_bwd_kernel<MODE, 4><<<grid, kNormThreads, 0, stream>>>(a);
   else gdpa_norm_rows_bwd_kernel<MODE, 8><<<grid, kNormThreads, 0, stream>>>(a);

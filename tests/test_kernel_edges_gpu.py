@@ -17,19 +17,15 @@ def G():
     return g
 
 
-@pytest.mark.parametrize("rows,n", [(1, 8), (3, 256), (37, 512), (300, 520), (1001, 1024), (29, 1032), (150, 2048), (7, 4096), (33, 4104)])
-@pytest.mark.parametrize("mode", [0, 1])
-def test_norm_backward_at_the_edges_of_its_row_lengths(mode, rows, n):
-    """Rows of 8 ... 4104 values (one to eight warps a row, then the kernel for longer rows), against autograd in fp64.
-    dx is a bf16 tensor: half an ulp, 2^-9 of the value; the sums in fp32 add some 1e-6 of the largest term.  The column
-    sums are fp32 over `rows` terms."""
+def _check_norm_backward(mode, rows, n, with_add, with_weight, want_dw, want_db):
+    """Against autograd in fp64.  dx is a bf16 tensor: half an ulp, 2^-9 of the value; the sums in fp32 add some 1e-6 of the
+    largest term.  The column sums are fp32 over `rows` terms."""
     from ads_model_kernel_library_b200.gdpa.megakernel import NORM_EPS, norm_rows_backward
 
     g = torch.Generator().manual_seed(rows + n)
     x, dy, add = (torch.randn(rows, 1, n, generator=g).to(torch.bfloat16) for _ in range(3))
     x = x + 0.5
-    w = 1 + 0.2 * torch.randn(n, generator=g)
-    want_dw = n <= 4096
+    w = 1 + 0.2 * torch.randn(n, generator=g) if with_weight else torch.ones(n)
     xd, wd, bd = x.double().view(rows, n).requires_grad_(True), w.double().requires_grad_(True), torch.zeros(n).double().requires_grad_(True)
     mean = xd.mean(1, keepdim=True)
     if mode == 0:
@@ -38,18 +34,44 @@ def test_norm_backward_at_the_edges_of_its_row_lengths(mode, rows, n):
     else:
         rstd = torch.rsqrt((xd - mean).square().mean(1, keepdim=True) + NORM_EPS)
         y = (xd - mean) * rstd * wd + bd
-    y.backward((dy.double() + (add.double() if mode == 1 else 0)).view(rows, n))
-    dx, dw, db = norm_rows_backward(mode, dy.cuda(), add.cuda() if mode == 1 else None, x.cuda(), w.cuda(),
+    y.backward((dy.double() + (add.double() if with_add else 0)).view(rows, n))
+    dx, dw, db = norm_rows_backward(mode, dy.cuda(), add.cuda() if with_add else None, x.cuda(), w.cuda() if with_weight else None,
                                     mean.detach().float().view(-1).cuda(), rstd.detach().float().view(-1).cuda(),
-                                    want_dweight=want_dw, want_dbias=want_dw and mode == 1)
+                                    want_dweight=want_dw, want_dbias=want_db)
     torch.cuda.synchronize()
     ref = xd.grad.view_as(dx)
     assert ((dx.cpu().double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all()
+    assert (dw is None) == (not want_dw) and (db is None) == (not want_db)
+    tol = 1e-6 * rows ** 0.5 * 16 + 1e-5  # fp32 sums of terms of a few units
     if want_dw:
-        tol = 1e-6 * rows ** 0.5 * 16 + 1e-5  # fp32 sums of terms of a few units
         assert ((dw.cpu().double() - wd.grad).abs() <= tol * (1 + wd.grad.abs())).all()
-        if mode == 1:
-            assert ((db.cpu().double() - bd.grad).abs() <= tol * (1 + bd.grad.abs())).all()
+    if want_db and mode == 1:
+        assert ((db.cpu().double() - bd.grad).abs() <= tol * (1 + bd.grad.abs())).all()
+
+
+@pytest.mark.parametrize("rows,n", [(1, 8), (3, 256), (37, 512), (300, 520), (1001, 1024), (29, 1032), (150, 2048), (7, 4096), (33, 4104)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_norm_backward_at_the_edges_of_its_row_lengths(mode, rows, n):
+    """Rows of 8 ... 4104 values: one to eight warps a row, then the kernel for longer rows."""
+    _check_norm_backward(mode, rows, n, mode == 1, True, n <= 4096, n <= 4096 and mode == 1)
+
+
+@pytest.mark.parametrize("rows,n", [(11003, 256), (5501, 1024), (2701, 2048), (1351, 4096)])
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("add,weight,dw,db", [(True, True, True, True), (False, True, True, False), (True, False, False, True)])
+def test_norm_backward_over_several_rounds_of_its_grid(mode, rows, n, add, weight, dw, db):
+    """Three full rounds and a part of one of 148 * 3 blocks (RMS norm; the layer norm has fewer blocks and more rounds), with
+    one, two, four and eight warps a row: the column sums are carried from round to round."""
+    _check_norm_backward(mode, rows, n, add, weight, dw, db and mode == 1)
+
+
+@pytest.mark.parametrize("rows,n", [(30001, 8), (24001, 64), (9001, 383), (9001, 384), (500, 768), (3000, 896), (3000, 904), (700, 1536),
+                                    (700, 1544), (900, 1792), (900, 1800), (300, 2560), (300, 3064), (300, 3072), (40, 8192)])
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("add,weight", [(True, True), (False, False)])
+def test_norm_backward_without_column_sums(mode, rows, n, add, weight):
+    """On both sides of the row lengths at which the kernel changes; the first rows take several rounds of the grid."""
+    _check_norm_backward(mode, rows, n // 8 * 8, add, weight, False, False)
 
 
 def _schedule(qo, ko, mode, heads, max_q, max_kv, kv_index=None):
