@@ -468,9 +468,13 @@ int launch_quant_fp8(const QuantArgs& a, int in_is_fp32, cudaStream_t stream) {
   gdpa_block_offsets_kernel<<<1, kScanThreads, 0, stream>>>(a.offsets, a.block_offsets, a.off64, a.batch);
   if (cudaGetLastError() != cudaSuccess) return GDPA_ERR_LAUNCH_;
   if (a.max_blocks == 0) return 0;
-  // the two head dims the forward takes; the other sizes, fp32 and unaligned tensors go through the general kernel, and so
-  // would more tiles than a 1-D grid holds
-  if (!in_is_fp32 && a.vec16 && (a.head_dim == 64 || a.head_dim == 128) && a.max_blocks * a.heads < (1ll << 31)) {
+  // The two head dims the forward takes; the other sizes, fp32 and unaligned tensors go through the general kernel, and so
+  // would more tiles than a 1-D grid holds, and batches whose sequences have fewer than 80 rows on average: with a few rows
+  // a tile the time is that of a CTA's dependent loads, and three times as many of the general kernel's CTAs are resident
+  // (524 288 rows of 4 heads of 128 in sequences of 8 rows 1630 us here and 1001 us there, of 64 rows 295 and 280, of 96 rows
+  // 260 and 263, of 2000 rows 190 and 229).
+  if (!in_is_fp32 && a.vec16 && (a.head_dim == 64 || a.head_dim == 128) && a.max_blocks * a.heads < (1ll << 31) &&
+      a.total >= 80ll * a.batch) {
     const unsigned tiles = static_cast<unsigned>(a.max_blocks * a.heads);
     if (a.head_dim == 64) gdpa_quant_fp8_tile_kernel<64><<<tiles, kQuantThreads, 0, stream>>>(a);
     else gdpa_quant_fp8_tile_kernel<128><<<tiles, kQuantThreads, 0, stream>>>(a);

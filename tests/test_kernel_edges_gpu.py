@@ -227,34 +227,45 @@ def test_shared_kv_result_does_not_depend_on_the_sequences_beside_it(G, act):
 
 
 @pytest.mark.parametrize("D", [64, 128])
-def test_fp8_quantiser_rounds_as_a_division(G, D):
-    """The one-pass quantiser against the restatement, byte for byte: ragged blocks, more sequences than one round of the
-    owner search holds, zeros, denormals, a block with an infinity, a NaN, and every bf16 mantissa over many scales."""
+@pytest.mark.parametrize("long", [0, 9000])
+def test_fp8_quantiser_rounds_as_a_division(G, D, long):
+    """Both kernels (the one-pass kernel takes batches of 80 rows a sequence and more: those with a long sequence added) against
+    the restatement, byte for byte: ragged blocks, more sequences than one round of the owner search holds, zeros, denormals,
+    blocks at the 1e-12 scale, infinities and NaN, and every bf16 mantissa over many scales.  A NaN does not count for the scale
+    of its block; NaN and, their scale being infinite, infinities become -448."""
     g = torch.Generator().manual_seed(D)
-    lens = [130, 0, 1, 128, 127, 384] + [5, 0, 3] * 20
+    lens = [130, 0, 1, 128, 127, 384] + [5, 0, 3] * 20 + [128, 128, long]
     off = torch.tensor(np.concatenate([[0], np.cumsum(lens)]))
     T, H = int(off[-1]), 3
+    assert (T >= 80 * len(lens)) == (long > 0)
     x = (torch.randn(T, H, D, generator=g) * torch.exp2(torch.randint(-30, 30, (T, H, 1), generator=g).float())).to(torch.bfloat16)
     x[0:131, 0] = 0
     x[131:140, 1] = 1e-39
     x[260:300, 2, 3] = float("inf")
+    x[300:310, 2, 5] = -float("inf")
+    x[131:200, 2, 7] = float("nan")
+    at = int(off[-4])  # two whole tiles
+    x[at:at + 128] = 1e-39
+    x[at + 128:at + 256] = ((torch.rand(128, H, D, generator=g) * 2 - 1) * 4e-10).to(torch.bfloat16)
     x8, sc, bo = G.quantize_fp8_blockwise(x.cuda(), off.cuda())
     torch.cuda.synchronize()
-    r8, rsc, rbo = orc.quantize_fp8_blockwise(x, off)
+    r8, rsc, rbo = orc.quantize_fp8_blockwise(x.nan_to_num(0, float("inf"), -float("inf")), off)
     assert torch.equal(bo.cpu(), rbo.to(bo.dtype)) and torch.equal(sc.cpu()[: rsc.shape[0]], rsc)
-    same = x8.cpu().view(torch.uint8) == r8.view(torch.uint8)
-    same |= ~torch.isfinite(x.float())  # inf / inf is a NaN: the restatement's clamp keeps it, the kernels give -448
-    assert same.all()
-    n = 1 << 20  # the quotients themselves, scales of every mantissa
+    want = torch.where(x.isfinite(), r8.view(torch.uint8), torch.full_like(r8, -448.0).view(torch.uint8))
+    assert torch.equal(x8.cpu().view(torch.uint8), want)
+    assert bool((rsc[int(rbo[-4]):int(rbo[-2])] == 1e-12).all()) and len(want[at + 128:at + 256].unique()) > 100
+    n = 1 << 20  # the quotients themselves, scales of every mantissa: one-row sequences, a scale per row
     amax = (torch.randint(0x3F80, 0x4000, (n // 128,), generator=g).to(torch.int16).view(torch.bfloat16)).float()
     v = (torch.rand(n // 128, 128, generator=g) * 2 - 1) * amax[:, None]
     v[:, 0] = amax
     y = v.to(torch.bfloat16).view(-1, 1, 128)
-    yo = torch.arange(0, n // 128 + 1)  # one-row sequences: a scale per row
-    y8, _, _ = G.quantize_fp8_blockwise(y.cuda(), yo.cuda())
+    rows = n // 128
+    yo = torch.cat([torch.arange(0, rows + 1), torch.tensor([81 * rows])]) if long else torch.arange(0, rows + 1)
+    padded = torch.cat([y, torch.zeros(80 * rows, 1, 128, dtype=y.dtype)]) if long else y
+    y8, _, _ = G.quantize_fp8_blockwise(padded.cuda(), yo.cuda())
     scale = (y.float().abs().amax(2, keepdim=True) / 448).clamp_min(1e-12)
     want = (y.float() / scale).clamp(-448, 448).to(torch.float8_e4m3fn)
-    assert torch.equal(y8.cpu().view(torch.uint8), want.view(torch.uint8))
+    assert torch.equal(y8[:rows].cpu().view(torch.uint8), want.view(torch.uint8))
 
 
 @pytest.mark.parametrize("D", [64, 128])
