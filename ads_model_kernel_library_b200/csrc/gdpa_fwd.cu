@@ -571,10 +571,12 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
           if (j == 0) {
             m_used = m_new;
           } else if (__any_sync(0xffffffffu, m_new > m_used + kThr)) {
-            // a row that has not seen a key yet (both maxima -inf) keeps its zeros
-            const float alpha = (m_new == -INFINITY) ? 1.f : ex2_approx(m_used - m_new);
+            // The rows of a warp move their maxima together.  In a run of sequences each row moves its own, so that no row's
+            // rounding depends on another sequence.  A row that has not seen a key yet (both maxima -inf) keeps its zeros.
+            const bool stays = !FP8 && m_new <= m_used + kThr && a.sched[1] == kSchedFwdShared;
+            const float alpha = (m_new == -INFINITY || stays) ? 1.f : ex2_approx(m_used - m_new);
             row_sum *= alpha;
-            m_used = m_new;
+            if (!stays) m_used = m_new;
 #pragma unroll
             for (int ch = 0; ch < D / 64; ++ch) {
               uint32_t ro[32];

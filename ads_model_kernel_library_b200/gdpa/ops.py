@@ -471,12 +471,10 @@ def _gdpa_forward_shared_kv_op(
         o = torch.empty(query.shape, dtype=query.dtype, device=query.device)
         if query.shape[0] == 0 or batch == 0:
             return o
-        # An element-wise activation without a band: a row's result depends neither on its position nor on the rows
-        # beside it, so neighbouring Q sequences of one KV sequence are scheduled as one.  (The softmax moves the
-        # reference maximum of a warp's 32 rows together; a sequence's rounding would depend on its neighbours.)
-        runs = window_size < 0 and activation != SOFTMAX_ID
-        sched = _build_schedule(_cabi.GDPA_SCHED_FWD_SHARED_KV if runs else _cabi.GDPA_SCHED_FWD, query_offset, key_offset,
-                                batch, H, query.shape[0], max_seq_len_q, max_seq_len_kv, kv_index)
+        # Without a band a row's result does not depend on its position, nor on the rows beside it (in a run the softmax
+        # keeps a reference maximum for every row): neighbouring Q sequences of one KV sequence are scheduled as one.
+        sched = _build_schedule(_cabi.GDPA_SCHED_FWD if window_size >= 0 else _cabi.GDPA_SCHED_FWD_SHARED_KV, query_offset,
+                                key_offset, batch, H, query.shape[0], max_seq_len_q, max_seq_len_kv, kv_index)
         p = _fill_fwd_params(query, key, value, o, query_offset, key_offset, batch, H, D, max_seq_len_q,
                              max_seq_len_kv, qk_scale, activation, sched, _cabi.GDPA_DTYPE_BF16)
         p.kv_seq_index = kv_index.data_ptr()

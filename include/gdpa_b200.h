@@ -95,8 +95,8 @@ enum {
   /* Forward with kv_seq_index and no window: neighbouring Q sequences that read the same KV sequence are taken
    * together, one work item per (run of sequences, head, 256- or 128-row Q block).  For gdpa_fwd only (not for
    * gdpa_fwd_fp8, whose scales are per sequence, and not for a call with a window, which counts positions in the
-   * sequence: there the kernel refuses it).  With GDPA_ACT_SOFTMAX the rounding of a sequence's rows then depends on
-   * the other sequences of its run; with the element-wise activations nothing does. */
+   * sequence: there the kernel refuses it).  The element-wise activations give the same bits as with GDPA_SCHED_FWD; the softmax
+   * rounds from another reference maximum, which is a row's own and depends on no other sequence. */
   GDPA_SCHED_FWD_SHARED_KV = 2
 };
 

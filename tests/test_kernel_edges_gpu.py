@@ -186,7 +186,9 @@ def test_shared_kv_runs_cover_every_row_once(requests, per, rows, heads):
 @pytest.mark.parametrize("per,rows", [(7, 20), (150, 90)])
 def test_shared_kv_runs_give_what_single_sequences_give(G, D, act, per, rows):
     """The same call with a band that reaches every pair is scheduled sequence by sequence.  A row's products, and the order
-    of its fp32 sums over the KV tiles, are the same in both: so are the results."""
+    of its fp32 sums over the KV tiles, are the same in both: so are the results.  Softmax: single sequences move the reference
+    maximum of 32 rows together and runs that of each row, so P is rounded to bf16 (2^-9) from another base; a weighted mean
+    of values of a unit then moves by less than that, and by an ulp of bf16, 2^-7 of its value, where it is rounded itself."""
     g = torch.Generator().manual_seed(per)
     rng = np.random.default_rng(per)
     requests, H = 3, 2
@@ -199,7 +201,10 @@ def test_shared_kv_runs_give_what_single_sequences_give(G, D, act, per, rows):
                                                window_size=w) for w in (None, 1 << 20)]
     torch.cuda.synchronize()
     assert G.kernel_status() == 0
-    assert torch.equal(out[0], out[1])
+    if act == "softmax":
+        assert_close(out[0], out[1], "runs", atol=2.0 ** -9, rtol=2.0 ** -7)
+    else:
+        assert torch.equal(out[0], out[1])
 
 
 @pytest.mark.parametrize("act", ["softmax", "silu", "relu"])
