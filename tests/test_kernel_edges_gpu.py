@@ -274,14 +274,17 @@ def test_fp8_quantiser_rounds_as_a_division(G, D, long):
 
 
 @pytest.mark.parametrize("D", [64, 128])
-def test_forward_of_items_of_one_to_three_ragged_kv_tiles(D):
+@pytest.mark.parametrize("repeat", [1, 10])
+def test_forward_of_items_of_one_to_three_ragged_kv_tiles(D, repeat):
     """The loader asks for all tiles of an item of one or two KV tiles before it zeroes the ragged ones: every combination
-    of Q and KV lengths around one and two tiles, against fp64 within the bf16 bound of the kernels."""
+    of Q and KV lengths around one and two tiles, against fp64 within the bf16 bound of the kernels.  160 items, at most two
+    for each of 148 CTAs; ten times as many take a CTA twice around its ring of work items, from items of three KV tiles
+    to those of two and one."""
     import ads_model_kernel_library_b200.gdpa as G
 
     g = torch.Generator().manual_seed(D)
     edges = [1, 127, 128, 129, 255, 256, 257, 300]
-    lq, lk = [a for a in edges for _ in edges], [b for _ in edges for b in edges]
+    lq, lk = [a for a in edges for _ in edges] * repeat, [b for _ in edges for b in edges] * repeat
     qo, ko = (torch.tensor(np.concatenate([[0], np.cumsum(n)])) for n in (lq, lk))
     q = torch.randn(int(qo[-1]), 2, D, generator=g).to(torch.bfloat16)
     k, v = (torch.randn(int(ko[-1]), 2, D, generator=g).to(torch.bfloat16) for _ in range(2))
