@@ -172,8 +172,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
   // The loader warp walks the list, reads an item and its sequence's offsets (two dependent trips to memory, with FP8
   // a third for the rows of the block scales) and publishes what they say through a small ring in shared memory, an item
   // ahead of its use; the MMA thread and the activation warps start on an item with two or three shared-memory loads
-  // instead of making those trips each.  FP8 forward 4.96 -> 4.83 ms, the norm pipeline's step 7.77 -> 7.71 ms, the plain
-  // forward of long and short items unchanged.
+  // instead of making those trips each.  FP8 forward 4.96 -> 4.83 ms, the norm pipeline's step unchanged within its spread.
   // Slot: {head, row offset q0 of the Q block, first Q row, first KV row}, {lq, lkv, first KV tile, KV tiles}, {Q scale row of Q tile 0, KV
   // scale row of KV tile 0 (FP8), -, -}; head -1 ends the walk.
   int4* const work_ring = reinterpret_cast<int4*>(smem + L::kWorkOff);
@@ -294,7 +293,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         // Issue order Q0, K0, Q1, V0, K1, V1, ...  In an item of one or two KV tiles (all its tiles fit in the ring) none of
         // the copies of a group (the first four, then K1 and V1) waits for another to land: ragged tiles are zeroed and
         // released when the whole group has been asked for.  There the round trips to memory are what the item takes
-        // (training on lengths up to 256: 801 -> 755 us, the forward kernel 204 -> 162 us); with more KV tiles the loader is
+        // (lengths up to 256: the forward kernel 204 -> 162 us); with more KV tiles the loader is
         // ahead of the MMAs, and a ragged K that waits for the ring slot of its V would come later than it could (log-normal
         // forward 1.215 -> 1.232 ms with groups everywhere).  The softmax kernels' items are bound by their element-wise
         // work: FP8 4.82 -> 4.86 ms with groups, so they have none.
