@@ -370,15 +370,19 @@ __global__ void __launch_bounds__(kTile) gdpa_quant_fp8_kernel(const QuantArgs a
 // rows.  x / scale: with the correctly rounded r = 1 / scale, q = x r and the exact remainder x - q scale,
 // q + remainder r is the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990), two fused operations a value
 // in place of a division; the exponents cannot leave the normal range where the result is not zero, because
-// scale >= 1e-12 and |x| <= 448 scale (1 + 2^-23).  A block that holds an infinity has an infinite scale and divides.
-// Reading the tile twice in 16-value pieces took 472 us for 1 143 311 tokens of 4 heads of 128 (264 us at the copy rate);
-// quantising Q, K, V and the FP8 forward of that batch: 5.34 -> 5.12 ms.  (A persistent grid that finds the next tile's
-// rows while the current one is on its way was no faster than the old kernel: 457 us.)
+// scale >= 1e-12 and |x| <= 448 scale (1 + 2^-23).  A block that holds an infinity has an infinite scale and divides, and so
+// does one that holds a NaN.
+// What keeps it from the copy rate is that a CTA waits for the offsets, reads, finds the maximum, converts and writes one
+// after the other, so it needs as many CTAs as fit and little arithmetic between their phases: maxima as integers (a NaN
+// shows in them, and the values of a block without one need no test), packed products.  1 143 311 tokens of 4 heads of 128
+// (264 us at the copy rate): 394 us with a maximum and a clamp in floating point, 375 us without them in 80 registers (three
+// CTAs an SM), 327 us in 64 (four), 340 us in 48 (five, with spills); reading the tile twice in 16-value pieces 472 us;
+// a CTA that takes four heads one after another, each read under the one before, 388 us.
 constexpr int kQuantThreads = 256;
 template <int D>
-__global__ void __launch_bounds__(kQuantThreads) gdpa_quant_fp8_tile_kernel(const QuantArgs a) {
+__global__ void __launch_bounds__(kQuantThreads, 4) gdpa_quant_fp8_tile_kernel(const QuantArgs a) {
   constexpr int kPieces = D / 16, kPerRow = D / 8, kRowStep = kQuantThreads / kPerRow;
-  __shared__ float s_max[kQuantThreads / 32];
+  __shared__ uint32_t s_max[2][kQuantThreads / 32];
   const long long g = blockIdx.x / static_cast<unsigned>(a.heads);
   const int h = blockIdx.x % static_cast<unsigned>(a.heads);
   if (g >= load_offset(a.block_offsets, a.batch, a.off64)) return;
@@ -398,24 +402,42 @@ __global__ void __launch_bounds__(kQuantThreads) gdpa_quant_fp8_tile_kernel(cons
     const int row = row_first + i * kRowStep;
     raw[i] = row < nrows ? *reinterpret_cast<const uint4*>(x + row * stride + c) : make_uint4(0, 0, 0, 0);
   }
-  __nv_bfloat162 m2 = __floats2bfloat162_rn(0.f, 0.f);
+  // maxima of |x| as integers: the bits of non-negative bf16 are in the order of their values, a NaN's above infinity's
+  uint32_t m2 = 0;
 #pragma unroll
   for (int i = 0; i < kPieces; ++i) {
     const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[j])));
+    for (int j = 0; j < 4; ++j) m2 = max_u16x2(m2, w[j] & 0x7fff7fffu);
   }
-  float amax = fmaxf(__low2float(m2), __high2float(m2));
+  auto block_max = [&](uint32_t v, uint32_t* slots) -> uint32_t {
+    v = __reduce_max_sync(0xffffffffu, v);
+    if ((t & 31) == 0) slots[t >> 5] = v;
+    __syncthreads();
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
-  if ((t & 31) == 0) s_max[t >> 5] = amax;
-  __syncthreads();
+    for (int i = 0; i < kQuantThreads / 32; ++i) v = max(v, slots[i]);
+    return v;
+  };
+  uint32_t amax_bits = block_max(max(m2 & 0xffffu, m2 >> 16), s_max[0]);
+  const bool has_nan = amax_bits > 0x7f80u;  // the same for the whole block
+  if (has_nan) {  // the maximum without them
+    uint32_t m = 0;
 #pragma unroll
-  for (int i = 0; i < kQuantThreads / 32; ++i) amax = fmaxf(amax, s_max[i]);
-  const float scale = fmaxf(amax / 448.f, 1e-12f);
+    for (int i = 0; i < kPieces; ++i) {
+      const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t lo = w[j] & 0x7fffu, hi = (w[j] >> 16) & 0x7fffu;
+        m = max(m, max(lo > 0x7f80u ? 0u : lo, hi > 0x7f80u ? 0u : hi));
+      }
+    }
+    amax_bits = block_max(m, s_max[1]);
+  }
+  const float scale = fmaxf(__uint_as_float(amax_bits << 16) / 448.f, 1e-12f);
   if (t == 0) a.scales[g * a.heads + h] = scale;
   const float inv = 1.f / scale;
-  const bool finite = scale <= 3.4028234664e38f;
+  const bool plain = !has_nan && amax_bits < 0x7f80u;
+  const uint64_t inv2 = pack_f32x2(inv, inv), neg_scale2 = pack_f32x2(-scale, -scale);
 #pragma unroll
   for (int i = 0; i < kPieces; ++i) {
     const int row = row_first + i * kRowStep;
@@ -424,19 +446,16 @@ __global__ void __launch_bounds__(kQuantThreads) gdpa_quant_fp8_tile_kernel(cons
     float v[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      v[2 * j] = __uint_as_float(w[j] << 16);
-      v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (finite) {
-        const float q = v[j] * inv;
-        v[j] = fmaf(fmaf(-q, scale, v[j]), inv, q);
+      const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xffff0000u);
+      if (plain) {
+        const uint64_t x2 = pack_f32x2(lo, hi), q = mul_f32x2(x2, inv2);
+        unpack_f32x2(fma_f32x2(fma_f32x2(q, neg_scale2, x2), inv2, q), v[2 * j], v[2 * j + 1]);
       } else {
-        v[j] = v[j] / scale;
+        v[2 * j] = fmaxf(lo / scale, -448.f);  // also what a NaN becomes
+        v[2 * j + 1] = fmaxf(hi / scale, -448.f);
       }
-      v[j] = fmaxf(v[j], -448.f);  // also what a NaN becomes; the conversion saturates at +448
     }
+    // the conversion saturates at +-448
     *reinterpret_cast<uint2*>(x8 + row * stride + c) =
         make_uint2(pack_e4m3x4(v[0], v[1], v[2], v[3]), pack_e4m3x4(v[4], v[5], v[6], v[7]));
   }

@@ -1,0 +1,31 @@
+"""FP8 block quantiser: blocks that hold NaN, infinities, both, or nothing else, byte for byte."""
+import pytest
+import torch
+
+from oracle import gdpa_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_blocks_with_nan_and_infinity(head_dim):
+    """One sequence of six blocks, the last of one row; a NaN (either sign, the smallest payload and the largest) does not count
+    for its block's scale and becomes -448, as does everything of a block whose scale is infinite and that is not finite."""
+    import ads_model_kernel_library_b200.gdpa as G
+
+    off = torch.tensor([0, 641])
+    g = torch.Generator().manual_seed(head_dim)
+    x = torch.randn(641, 3, head_dim, generator=g).to(torch.bfloat16)
+    bits = x.view(torch.int16)
+    bits[3, 0, 0], bits[127, 0, head_dim - 1] = 0x7F81, -1  # block 0, head 0: two NaN among finite values
+    bits[130, 1, 5], x[200, 1, 9] = 0x7FFF, float("inf")  # block 1, head 1: NaN and infinity
+    bits[256:384, 2] = 0x7FC0  # block 2, head 2: NaN only
+    x[400, 0, 1] = -float("inf")  # block 3, head 0
+    bits[640, 1, 0] = 0x7FC0  # block 5, a single row
+    x[640, 2] = 0
+    x8, scales, blocks = G.quantize_fp8_blockwise(x.cuda(), off.cuda())
+    # a NaN as 0 gives the scale without it
+    r8, rscales, rblocks = orc.quantize_fp8_blockwise(x.nan_to_num(0, float("inf"), -float("inf")), off)
+    want = torch.where(x.isfinite(), r8.view(torch.uint8), torch.tensor(0xFE, dtype=torch.uint8))  # 0xFE: -448
+    assert torch.equal(blocks.cpu(), rblocks) and torch.equal(scales.cpu()[:6], rscales)
+    assert torch.equal(x8.cpu().view(torch.uint8), want)
