@@ -27,7 +27,7 @@
 //
 // Roles (16 warps, setmaxnreg 144 / 144 / 80): warps 0-3 dQ reduce, warps 4-11 element-wise (warp w:
 // TMEM lanes 32*(w%4), score columns 64*((w-4)/4); at the end of a work item they write dK and dV out through their own
-// part of the dS^T buffer), warp 12 MMA issuer (one lane), warp 13 TMA loader (lane 0 issues the copies and draws the
+// part of the dS^T buffer), warp 12 MMA issuer (one elected thread), warp 13 TMA loader (lane 0 issues the copies and draws the
 // work items, the warp zeroes the tails of ragged tiles), warps 14-15 idle.
 // P^T of column half h is written over the first 32 columns of that half's own S^T columns
 // ([64h, 64h+32)), so the two halves never touch each other's unread scores.
@@ -76,7 +76,7 @@ enum BwdBar : int {
   BB_ST_FULL = 18,  // 256 arrivals: softmax, the per-column statistics of a Q tile are in shared memory
   BB_LD_TMP = 19,   // the loader's own: a ragged tile has landed and can have its padding rows zeroed
   BB_WORK_FULL = 20,   // [kWorkSlots] the loader has published the index of a work item
-  BB_WORK_EMPTY = 24,  // [kWorkSlots] 13 arrivals: the MMA thread, 8 element-wise and 4 drain warps have read it
+  BB_WORK_EMPTY = 24,  // [kWorkSlots] 13 arrivals: the MMA warp, 8 element-wise and 4 drain warps have read it
   BB_COUNT = 28
 };
 constexpr int kWorkSlots = 4;
@@ -110,11 +110,8 @@ struct BwdSmem {
 // parities as bits of one word, operand descriptors built once per role) and full tiles take a path with no test
 // per MMA.
 
-#define GDPA_WAIT(bar_idx, parity, role)                                                                   \
-  if (!mbar_wait(bar_base + 8u * (bar_idx), (parity), abort_flag, a.status, ((bar_idx) << 8) | (role))) \
-    goto role_done;
-// The same for roles whose whole warp waits and then executes warp-collective tcgen05.ld / st: the
-// decision to leave is taken by the warp as a whole, so no lane runs ahead into a collective instruction.
+// Every role waits as a whole warp: the decision to leave is the warp's, so no lane runs ahead into a collective instruction
+// (tcgen05.ld / st, the vote for the thread that issues the MMAs).
 #define GDPA_WAIT_WARP(bar_idx, parity, role)                                                                       \
   {                                                                                                                 \
     const bool ok_ = mbar_wait(bar_base + 8u * (bar_idx), (parity), abort_flag, a.status, ((bar_idx) << 8) | (role)); \
@@ -136,7 +133,7 @@ gdpa_bwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
   volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(smem + L::kTmemPtrOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kAbortOff);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -164,7 +161,7 @@ gdpa_bwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
   const int n_items = schedule_items(a.sched, a.sched[1] == kSchedBwd, a.status);
   const SeqLimits lim = {a.total_q, a.total_kv, 0};
 #ifdef GDPA_ENABLE_TRACE
@@ -181,18 +178,18 @@ gdpa_bwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
   int* const work_counter = const_cast<int*>(a.sched) + 3;
   uint32_t work_pos = 0;  // items this role has taken: ring slot = work_pos % kWorkSlots, parity = (work_pos / kWorkSlots) & 1
   // Consumer side: the index of this role's next work item, -1 at the end of the list, -2 if the wait ran out.
-  // `warp_wide`: called by a whole warp, whose lane 0 releases the slot.  (A function that is not inlined would keep
+  // Called by a whole warp, whose lane 0 releases the slot.  (A function that is not inlined would keep
   // this out of the roles' code, but register allocation fails for calls in a kernel with fixed register counts.)
-  auto take_work_item = [&](int role, bool warp_wide) -> int {
+  auto take_work_item = [&](int role) -> int {
     const uint32_t slot = work_pos % kWorkSlots, parity = (work_pos / kWorkSlots) & 1u;
     ++work_pos;
     bool ok = mbar_wait(bar_base + 8u * (BB_WORK_FULL + slot), parity, abort_flag, a.status, ((BB_WORK_FULL + slot) << 8) | role);
-    if (warp_wide) ok = __all_sync(0xffffffffu, ok);
+    ok = __all_sync(0xffffffffu, ok);
     if (!ok) return -2;
     int idx;
     asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(idx) : "r"(work_ring + 4u * slot) : "memory");
-    if (warp_wide) __syncwarp();
-    if (!warp_wide || lane == 0) mbar_arrive(bar_base + 8u * (BB_WORK_EMPTY + slot));
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar_base + 8u * (BB_WORK_EMPTY + slot));
     return idx;
   };
 
@@ -322,7 +319,11 @@ gdpa_bwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
       }
     } else if (warp == kBwdMmaWarp) {
       // ---------------------------------------------------------------- MMA issuer
-      if (lane == 0) {
+      // The whole warp walks the loop, with bounds and stages that are the same for its lanes, and one elected thread issues:
+      // the operands stay in uniform registers.  As one lane's code under a branch: 8.85 -> 8.40 ms on 128 sequences of 512 to
+      // 4096 tokens of 8 heads, the softmax's 1063 -> 1027 us.  (In that form a rolled loop of the slices cost 13 %, two issuing
+      // warps, one for S^T and dV and one for dP^T, dK and dQ, 16 %.)
+      {
         uint32_t kv_phase = 0, q_phase = 0 /* bit st = parity of Q stage st */, do_phase = 0, st = 0;
         uint32_t p_phase = 0, ds_phase = 0, dqe_phase = 0, dkve_phase = 0;
         int tr = 0;  // trace: Q tiles seen so far (slot layout: tr * 32 + event, events 0-7 MMA, 8-12 element-wise, 13-16 reduce)
@@ -345,21 +346,21 @@ gdpa_bwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         };
         int idx;
         while (true) {
-          idx = take_work_item(ST_ROLE_MMA, false);
+          idx = warp_uniform(take_work_item(ST_ROLE_MMA));
           if (idx == -2) goto role_done;
           if (idx < 0) break;
           const Work w = load_work(a.sched, idx, a.q_off, a.kv_off, a.off64, a.max_q, a.max_kv, lim);
           int m0, nq1;
           bwd_q_range(w, a.window, m0, nq1);
-          const int nq = nq1 * a.kv_group;
+          const int nq = warp_uniform(nq1 * a.kv_group);
           if (nq == 0) continue;
-          GDPA_WAIT(BB_KV_FULL, kv_phase, ST_ROLE_MMA);
+          GDPA_WAIT_WARP(BB_KV_FULL, kv_phase, ST_ROLE_MMA);
           kv_phase ^= 1u;
           for (int m = 0; m <= nq; ++m) {
             const uint64_t dQ_k = umma_desc_advance(dQ0_k, st * L::kTileBytes);
             if (m < nq) {
               GDPA_TRACE(a, tr * 32 + 0);
-              GDPA_WAIT(BB_Q_FULL + st, (q_phase >> st) & 1u, ST_ROLE_MMA);
+              GDPA_WAIT_WARP(BB_Q_FULL + st, (q_phase >> st) & 1u, ST_ROLE_MMA);
               q_phase ^= 1u << st;
               tc_fence_after();
               mma_kmajor_pair(kColS, dK_k, dQ_k);  // S^T = K Q_m^T
@@ -369,7 +370,7 @@ gdpa_bwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
             if (m > 0) {
               const uint32_t pst = st ^ 1u;
               const uint64_t dQp_mn = umma_desc_advance(dQ0_mn, pst * L::kTileBytes);
-              GDPA_WAIT(BB_DS_FULL, ds_phase, ST_ROLE_MMA);
+              GDPA_WAIT_WARP(BB_DS_FULL, ds_phase, ST_ROLE_MMA);
               ds_phase ^= 1u;
               tc_fence_after();
               GDPA_TRACE(a, tr * 32 + 2);
@@ -390,20 +391,20 @@ gdpa_bwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
               GDPA_TRACE(a, tr * 32 + 3);
             }
             if (m < nq) {
-              GDPA_WAIT(BB_DO_FULL, do_phase, ST_ROLE_MMA);
+              GDPA_WAIT_WARP(BB_DO_FULL, do_phase, ST_ROLE_MMA);
               do_phase ^= 1u;
-              GDPA_WAIT(BB_DQ_EMPTY, dqe_phase ^ 1u, ST_ROLE_MMA);
+              GDPA_WAIT_WARP(BB_DQ_EMPTY, dqe_phase ^ 1u, ST_ROLE_MMA);
               dqe_phase ^= 1u;
               tc_fence_after();
               GDPA_TRACE(a, tr * 32 + 4);
               mma_kmajor_pair(kColDP, dV_k, dDo_k);  // dP^T = V dO_m^T
               tc_commit(bar_base + 8u * BB_DP_FULL);
               GDPA_TRACE(a, tr * 32 + 5);
-              GDPA_WAIT(BB_P_FULL, p_phase, ST_ROLE_MMA);
+              GDPA_WAIT_WARP(BB_P_FULL, p_phase, ST_ROLE_MMA);
               p_phase ^= 1u;
               GDPA_TRACE(a, tr * 32 + 6);
               if (m == 0) {
-                GDPA_WAIT(BB_DKV_EMPTY, dkve_phase ^ 1u, ST_ROLE_MMA);
+                GDPA_WAIT_WARP(BB_DKV_EMPTY, dkve_phase ^ 1u, ST_ROLE_MMA);
                 dkve_phase ^= 1u;
               }
               tc_fence_after();
@@ -444,7 +445,7 @@ gdpa_bwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
     const float c2 = a.scale * 1.4426950408889634f;
     int idx;
     while (true) {
-      idx = take_work_item(ST_ROLE_ACT, true);
+      idx = take_work_item(ST_ROLE_ACT);
       if (idx == -2) goto role_done;
       if (idx < 0) break;
       const Work w = load_work(a.sched, idx, a.q_off, a.kv_off, a.off64, a.max_q, a.max_kv, lim);
@@ -684,7 +685,7 @@ gdpa_bwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
     int tr = 0;
     int idx;
     while (true) {
-      idx = take_work_item(ST_ROLE_RED, true);
+      idx = take_work_item(ST_ROLE_RED);
       if (idx == -2) goto role_done;
       if (idx < 0) break;
       const Work w = load_work(a.sched, idx, a.q_off, a.kv_off, a.off64, a.max_q, a.max_kv, lim);
@@ -772,7 +773,6 @@ role_done:
   }
 }
 
-#undef GDPA_WAIT
 #undef GDPA_WAIT_WARP
 
 __global__ void __launch_bounds__(256) gdpa_dq_convert_kernel(const float4* __restrict__ acc, uint2* __restrict__ dq,

@@ -9,7 +9,7 @@
 //               item the same warps drain their half of O0 (TMEM -> bf16 -> a staging slab in shared memory ->
 //               TMA store).
 //   warps 8-15  the same for Q tile 1
-//   warp  16    MMA issuer (one lane): S_s = Q_s K^T (tcgen05.mma, operands in shared memory),
+//   warp  16    MMA issuer (one elected thread): S_s = Q_s K^T (tcgen05.mma, operands in shared memory),
 //               O_s += P_s V (A operand P read from TMEM)
 //   warp  17    TMA loader (lane 0 issues the copies, the warp zeroes the tails of ragged tiles);  warps 18-19 idle
 //
@@ -57,7 +57,7 @@ enum FwdBar : int {
   B_M_FULL = 14 + 2 * kKvStages,       // [2] softmax, wide layout: both column halves have published their row maxima
   B_LD_TMP = 16 + 2 * kKvStages,       // [4] the loader's own: a ragged tile has landed and can have its padding rows zeroed
   B_WORK_FULL = 20 + 2 * kKvStages,               // [kWorkSlots] the loader has published a work item
-  B_WORK_EMPTY = 20 + 2 * kKvStages + kWorkSlots, // [kWorkSlots] the MMA thread and the 16 activation warps have read it
+  B_WORK_EMPTY = 20 + 2 * kKvStages + kWorkSlots, // [kWorkSlots] the MMA warp and the 16 activation warps have read it
   B_COUNT = 20 + 2 * kKvStages + 2 * kWorkSlots
 };
 
@@ -92,11 +92,8 @@ struct FwdSmem {
   static constexpr int kDynBytes = kBytes + 1024;        // slack to align the base to 1024 bytes
 };
 
-#define GDPA_WAIT(bar_idx, parity, role)                                                                   \
-  if (!mbar_wait(bar_base + 8u * (bar_idx), (parity), abort_flag, a.status, ((bar_idx) << 8) | (role))) \
-    goto role_done;
-// The same for roles whose whole warp waits and then executes warp-collective tcgen05.ld / st: the
-// decision to leave is taken by the warp as a whole, so no lane runs ahead into a collective instruction.
+// Every role waits as a whole warp: the decision to leave is the warp's, so no lane runs ahead into a collective instruction
+// (tcgen05.ld / st, the vote for the thread that issues the MMAs).
 #define GDPA_WAIT_WARP(bar_idx, parity, role)                                                                       \
   {                                                                                                                 \
     const bool ok_ = mbar_wait(bar_base + 8u * (bar_idx), (parity), abort_flag, a.status, ((bar_idx) << 8) | (role)); \
@@ -141,7 +138,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
   volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(smem + L::kTmemPtrOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kAbortOff);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -166,12 +163,12 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
   const SeqLimits lim = {a.total_q, a.total_kv, a.kv_batch};
 
   // The loader warp walks the list, reads an item and its sequence's offsets (two dependent trips to memory, with FP8
   // a third for the rows of the block scales) and publishes what they say through a small ring in shared memory, an item
-  // ahead of its use; the MMA thread and the activation warps start on an item with two or three shared-memory loads
+  // ahead of its use; the MMA warp and the activation warps start on an item with two or three shared-memory loads
   // instead of making those trips each.  FP8 forward 4.96 -> 4.83 ms, the norm pipeline's step unchanged within its spread.
   // Slot: {head, row offset q0 of the Q block, first Q row, first KV row}, {lq, lkv, first KV tile, KV tiles}, {Q scale row of Q tile 0, KV
   // scale row of KV tile 0 (FP8), -, -}; head -1 ends the walk.
@@ -181,18 +178,18 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
     int h, q0, q_start, kv_start, lq, lkv, j0, nkv, q_scale0, kv_scale0;  // the block takes rows [q0, min(lq, q0 + 256))
   };
   // Consumer side: this role's next work item; h = -1 at the end of the list, -2 if the wait ran out.
-  // `warp_wide`: called by a whole warp, whose lane 0 releases the slot.
-  auto take_work_item = [&](int role, bool warp_wide) -> Item {
+  // Called by a whole warp, whose lane 0 releases the slot.
+  auto take_work_item = [&](int role) -> Item {
     const uint32_t slot = work_pos % kWorkSlots, parity = (work_pos / kWorkSlots) & 1u;
     ++work_pos;
     bool ok = mbar_wait(bar_base + 8u * (B_WORK_FULL + slot), parity, abort_flag, a.status, ((B_WORK_FULL + slot) << 8) | role);
-    if (warp_wide) ok = __all_sync(0xffffffffu, ok);
+    ok = __all_sync(0xffffffffu, ok);
     if (!ok) return Item{-2, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     const int4 u = work_ring[3 * slot], v = work_ring[3 * slot + 1];
     int4 x = make_int4(0, 0, 0, 0);
     if (FP8) x = work_ring[3 * slot + 2];
-    if (warp_wide) __syncwarp();
-    if (!warp_wide || lane == 0) mbar_arrive(bar_base + 8u * (B_WORK_EMPTY + slot));
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar_base + 8u * (B_WORK_EMPTY + slot));
     return Item{u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w, x.x, x.y};
   };
 
@@ -335,7 +332,13 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
     }
    } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // The tensor pipe's queue is short, so how fast this warp issues is how fast it runs.  The whole warp walks the loop,
+    // with bounds and stages that are the same for its lanes, and one elected thread issues: operands stay in uniform
+    // registers.  As one lane's code under a branch: log-normal forward 1002 -> 966 us, FP8 3.79 -> 3.66 ms, head_dim 64 with a
+    // band 430 -> 380 us, 14.0 -> 13.0 ms on 512 sequences of 512 to 4096 tokens of 8 heads.  (In that form a rolled loop of
+    // the slices cost 19 %.  Two issuing warps, one for each Q tile, cost 25 %: the Q tiles fall into step, both in the
+    // activation and then both on the tensor pipe, where one warp keeps them alternating.)
+    {
       uint32_t kv_stage = 0, kv_phase = 0;
       // bit s of q_phase / p_phase / o_phase = parity of that barrier of Q tile s (registers, not arrays indexed by s)
       uint32_t q_phase = 0, p_phase = 0, o_phase = 0;
@@ -371,7 +374,8 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         }
       };
       while (true) {
-        const Item w = take_work_item(ST_ROLE_MMA, false);
+        Item w = take_work_item(ST_ROLE_MMA);
+        w.h = warp_uniform(w.h), w.nkv = warp_uniform(w.nkv), w.lq = warp_uniform(w.lq), w.q0 = warp_uniform(w.q0);
         if (w.h < 0) {
           if (w.h == -2) goto role_done;
           break;
@@ -383,9 +387,9 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
         {
           const uint32_t k_stage = kv_stage;
           for (int s = 0; s < nst; ++s) {
-            GDPA_WAIT(B_Q_FULL + s, (q_phase >> s) & 1u, ST_ROLE_MMA);
+            GDPA_WAIT_WARP(B_Q_FULL + s, (q_phase >> s) & 1u, ST_ROLE_MMA);
             q_phase ^= 1u << s;
-            if (s == 0) GDPA_WAIT(B_KV_FULL + k_stage, kv_phase, ST_ROLE_MMA);
+            if (s == 0) GDPA_WAIT_WARP(B_KV_FULL + k_stage, kv_phase, ST_ROLE_MMA);
             tc_fence_after();
             issue_qk(s, k_stage);
             tc_commit(bar_base + 8u * (B_S_FULL + s));
@@ -400,21 +404,21 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
           if (++kv_stage == kKvStages) { kv_stage = 0; kv_phase ^= 1u; }
           const uint32_t k_stage = kv_stage, k_phase = kv_phase;  // K_{j+1}, valid if more
           if (more) { if (++kv_stage == kKvStages) { kv_stage = 0; kv_phase ^= 1u; } }
-          GDPA_WAIT(B_KV_FULL + v_stage, v_phase, ST_ROLE_MMA);
+          GDPA_WAIT_WARP(B_KV_FULL + v_stage, v_phase, ST_ROLE_MMA);
           for (int s = 0; s < nst; ++s) {
             GDPA_TRACE(a, tr * 32 + 16 + s * 4 + 0);
-            GDPA_WAIT(B_P_FULL + s, (p_phase >> s) & 1u, ST_ROLE_MMA);
+            GDPA_WAIT_WARP(B_P_FULL + s, (p_phase >> s) & 1u, ST_ROLE_MMA);
             GDPA_TRACE(a, tr * 32 + 16 + s * 4 + 1);
             p_phase ^= 1u << s;
             if (j == 0) {
-              GDPA_WAIT(B_O_EMPTY + s, ((o_phase >> s) & 1u) ^ 1u, ST_ROLE_MMA);
+              GDPA_WAIT_WARP(B_O_EMPTY + s, ((o_phase >> s) & 1u) ^ 1u, ST_ROLE_MMA);
               o_phase ^= 1u << s;
             }
             tc_fence_after();
             issue_pv(s, v_stage, j > 0);
             if (more) {
               if (s == 0) {
-                GDPA_WAIT(B_KV_FULL + k_stage, k_phase, ST_ROLE_MMA);
+                GDPA_WAIT_WARP(B_KV_FULL + k_stage, k_phase, ST_ROLE_MMA);
                 tc_fence_after();
               }
               issue_qk(s, k_stage);
@@ -444,7 +448,7 @@ gdpa_fwd_kernel(const __grid_constant__ TmapSet tm_q, const __grid_constant__ Tm
     uint32_t s_phase = 0, o_phase = 0;
     int tr = 0;
     while (true) {
-      const Item w = take_work_item(ST_ROLE_ACT, true);
+      const Item w = take_work_item(ST_ROLE_ACT);
       if (w.h < 0) {
         if (w.h == -2) goto role_done;
         break;
@@ -928,7 +932,6 @@ role_done:
   }
 }
 
-#undef GDPA_WAIT
 #undef GDPA_WAIT_WARP
 
 template <int D, int ACT, bool FP8, bool FUSE>
