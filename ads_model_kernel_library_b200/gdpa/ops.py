@@ -11,7 +11,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
-from typing import List, Optional, Tuple
+from typing import Callable, List, NamedTuple, Optional, Tuple
 
 import torch
 
@@ -257,25 +257,77 @@ def _fill_fwd_params(q, k, v, o, qo, ko, batch, H, D, max_q, max_kv, scale, act_
     return p
 
 
-_library = torch.library.Library("gdpa", "FRAGMENT")
 _below_autograd = getattr(torch._C, "_AutoDispatchBelowAutograd", None)  # private, as above: without it, the public form
 _untraced = getattr(torch, "_disable_dynamo", torch.compiler.disable)  # the first imports the compiler when it is used, not now
 
+# The operators belong to the process, not to this module: torch keeps the handle of an operator that it has once looked up
+# (torch.ops, graphs), and such a handle points to freed memory when the operator is taken out of the dispatcher.  They are
+# kept on torch's own namespace object, which outlives the modules of this package.
+_operators = vars(torch.ops.gdpa).setdefault("_operators", {})
+
+
+class _Functions(NamedTuple):
+    impl: Callable
+    fake: Callable
+    setup_context: Callable
+    backward: Callable
+
+
+class _Gradient(torch.autograd.Function):
+    """A call that needs a gradient: the operator below autograd, and its ``backward``."""
+
+    @staticmethod
+    def forward(ctx, functions, overload, *args):
+        ctx.functions = functions  # this call's own, should the operator get others before its backward
+        with _below_autograd():
+            output = overload(*args)
+        functions.setup_context(ctx, args, output)
+        return output
+
+    @staticmethod
+    def backward(ctx, *grads):
+        return (None, None, *ctx.functions.backward(ctx, *grads))
+
+
+class _Operator:
+    """A torch operator with a CUDA kernel, a fake kernel and a gradient, registered once.  Its kernels look up ``functions``
+    when they are called, so that they can be replaced."""
+
+    def __init__(self, name: str, schema: str, functions: _Functions):
+        self.schema = schema
+        self.functions = functions
+        self.library = torch.library.Library("gdpa", "FRAGMENT")
+        self.library.define(schema, tags=(torch.Tag.pt2_compliant_tag,))
+        overload = getattr(torch.ops.gdpa, name).default
+        defaults = tuple(a.default_value for a in overload._schema.arguments)
+
+        def autograd_kernel(*args):
+            if torch.is_grad_enabled():
+                for a in args:
+                    if isinstance(a, torch.Tensor) and a.requires_grad:
+                        return _Gradient.apply(self.functions, overload, *args, *defaults[len(args):])
+            with _below_autograd():
+                return overload(*args)
+
+        # the CUDA kernel is not traced into when it runs beneath a compiled caller
+        self.library.impl(name, _untraced(lambda *args: self.functions.impl(*args)), "CUDA")
+        torch.library.register_fake(f"gdpa::{name}", lambda *args: self.functions.fake(*args), lib=self.library)
+        if _below_autograd is None:
+            torch.library.register_autograd(f"gdpa::{name}", lambda ctx, *grads: self.functions.backward(ctx, *grads),
+                                            setup_context=lambda *args, **kwargs: self.functions.setup_context(*args, **kwargs),
+                                            lib=self.library)
+        else:
+            self.library.impl(name, autograd_kernel, "Autograd")
+
 
 def _define_op(schema: str, impl, fake, setup_context=None, backward=None) -> None:
-    """Define ``gdpa::<schema>`` with a CUDA kernel, a fake kernel and its gradient: what ``torch.library.custom_op`` and
-    ``register_autograd`` do, with a gradient kernel of its own in place of theirs.  An operator without ``backward`` has no
-    gradient: differentiating its outputs raises.
+    """Make ``gdpa::<schema>`` with these functions, as ``torch.library.custom_op`` and ``register_autograd`` would; an operator
+    that is there already (this module is run a second time) gets them in place of its own.  Without ``backward``
+    differentiating the outputs raises.
 
-    A call on a few short sequences is host time only, and more than half of it was the generic form's: forward and backward
-    of eight sequences 278 -> 220 us, the forward of four requests with shared KV, without a gradient, 60 -> 51 us."""
+    A call on a few short sequences is host time only, a fifth of it the generic form's with a gradient and a seventh
+    without: forward and backward of eight sequences 278 -> 220 us, the forward of four requests with shared KV 60 -> 51 us."""
     name = schema[:schema.index("(")]
-    _library.define(schema, tags=(torch.Tag.pt2_compliant_tag,))
-    op = getattr(torch.ops.gdpa, name).default
-    defaults = tuple(a.default_value for a in op._schema.arguments)
-    _library.impl(name, _untraced(impl), "CUDA")  # not traced into when it runs beneath a compiled caller
-    torch.library.register_fake(f"gdpa::{name}", fake, lib=_library)
-
     if backward is None:
         def setup_context(ctx, inputs, output):
             pass
@@ -283,27 +335,15 @@ def _define_op(schema: str, impl, fake, setup_context=None, backward=None) -> No
         def backward(ctx, *grads):
             raise RuntimeError(f"Trying to backward through gdpa::{name} but it has no gradient")
 
-    if _below_autograd is None:
-        torch.library.register_autograd(f"gdpa::{name}", backward, setup_context=setup_context, lib=_library)
-        return
-
-    def forward(ctx, *args):
-        with _below_autograd():
-            out = op(*args)
-        setup_context(ctx, args, out)
-        return out
-
-    function = type(f"_{name}", (torch.autograd.Function,), {"forward": staticmethod(forward), "backward": staticmethod(backward)})
-
-    def autograd_kernel(*args):
-        if torch.is_grad_enabled():
-            for a in args:
-                if isinstance(a, torch.Tensor) and a.requires_grad:
-                    return function.apply(*args, *defaults[len(args):])
-        with _below_autograd():
-            return op(*args)
-
-    _library.impl(name, autograd_kernel, "Autograd")
+    functions = _Functions(impl, fake, setup_context, backward)
+    operator = _operators.get(name)
+    if operator is None:
+        _operators[name] = _Operator(name, schema, functions)
+    elif operator.schema == schema:
+        operator.functions = functions
+    else:
+        raise RuntimeError(f"gdpa::{name} is registered in this process with another schema, which cannot be taken back: "
+                           "start a new process")
 
 
 def _gdpa_forward(
@@ -883,9 +923,11 @@ def _register_flop_formulas() -> None:
     (gdpa/triton/triton_generalized_dot_product_attention.py:4051, :4137): 4 H D sum(Lq Lkv) forward,
     2.5x that backward, valid jagged pairs only."""
     try:
-        from torch.utils.flop_counter import register_flop_formula
+        from torch.utils.flop_counter import flop_registry, register_flop_formula
     except ImportError:  # pragma: no cover
         return
+    for packet in (torch.ops.gdpa.generalized_dot_product_attention, torch.ops.gdpa.generalized_dot_product_attention_backward):
+        flop_registry.pop(packet, None)  # there when this module is run a second time
 
     @register_flop_formula(torch.ops.gdpa.generalized_dot_product_attention, get_raw=True)
     def _fwd_flops(query, key, value, query_offset, key_offset, max_seq_len_q, max_seq_len_kv, *args, **kwargs) -> int:

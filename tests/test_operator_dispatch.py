@@ -119,3 +119,82 @@ for act in ("relu", "softmax"):
     assert torch.autograd.grad(out, q, torch.empty_like(out))[0].shape == q.shape
 """
     subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT, timeout=300)
+
+
+_SECOND_LOAD = """
+import importlib, sys
+import torch
+from torch.utils.flop_counter import FlopCounterMode
+import ads_model_kernel_library_b200.gdpa as G
+
+NAME = "ads_model_kernel_library_b200"
+
+def tensors():
+    q = torch.empty(10, 4, 64, dtype=torch.bfloat16, device="meta", requires_grad=True)
+    k = torch.empty(12, 2, 64, dtype=torch.bfloat16, device="meta", requires_grad=True)
+    return q, k, torch.empty(3, dtype=torch.int64, device="meta")
+
+def calls(attention, megakernel, fp8):
+    q, k, off = tensors()
+    for act in ("relu", "softmax"):
+        with FlopCounterMode(display=False) as flops:
+            out = attention(q, k, k, off, off, 5, 6, activation=act)
+            grads = torch.autograd.grad(out, (q, k), torch.empty_like(out))
+        assert [g.shape for g in grads] == [q.shape, k.shape]
+        assert flops.get_total_flops() == (14 if act == "relu" else 10) * 4 * 64 * 2 * 5 * 6  # the softmax forward has no formula
+        with torch.no_grad():
+            assert attention(q, k, k, off, off, 5, 6, activation=act).shape == q.shape
+    out = attention(q, k, k, off, off, 5, 6, activation="relu", ad_to_request_offset=off[:2])
+    try:
+        torch.autograd.grad(out, q, torch.empty_like(out))
+    except NotImplementedError as e:
+        assert "inference path" in str(e)
+    else:
+        raise AssertionError
+    out = megakernel(q, k, k, off, off, 5, 6, activation="relu", fused_rms_norm=True)
+    assert out.shape == q.shape and out.requires_grad
+    q8 = torch.empty(10, 2, 64, dtype=torch.float8_e4m3fn, device="meta")
+    s8 = torch.empty(2, 2, device="meta")
+    out = fp8(q8, q8, q8, s8, s8, s8, off, off, off, off, 5, 5)
+    assert out.shape == q8.shape and out.dtype == torch.bfloat16
+
+first = G.generalized_dot_product_attention, G.gdpa_megakernel, G.generalized_dot_product_attention_fp8
+overload = torch.ops.gdpa.generalized_dot_product_attention.default
+calls(*first)
+q, k, off = tensors()
+pending = {act: first[0](q, k, k, off, off, 5, 6, activation=act) for act in ("relu", "softmax")}
+for _ in range(2):
+    if HOW == "reload":
+        for module in ("ops", "megakernel", "mxfp8"):
+            importlib.reload(sys.modules[f"{NAME}.gdpa.{module}"])
+        importlib.reload(G)
+    else:
+        for module in [m for m in sys.modules if m.split(".")[0] == NAME]:
+            del sys.modules[module]
+        import ads_model_kernel_library_b200.gdpa as G
+    assert G.generalized_dot_product_attention is not first[0]
+    calls(G.generalized_dot_product_attention, G.gdpa_megakernel, G.generalized_dot_product_attention_fp8)
+    calls(*first)
+    assert overload(q, k, k, off, off, 5, 6, 1.0, 3).shape == q.shape
+for out in pending.values():
+    assert torch.autograd.grad(out, k, torch.empty_like(out))[0].shape == k.shape
+# a call reaches the functions of the module that was run last
+ops = sys.modules[f"{NAME}.gdpa.ops"]
+assert torch.ops.gdpa._operators["generalized_dot_product_attention"].functions.impl is ops._gdpa_forward
+"""
+
+
+@pytest.mark.parametrize("how", ["reload", "import"])
+def test_operators_outlive_a_second_load_of_their_module(how):
+    """importlib.reload, and an import after the package was taken out of sys.modules: calls, gradients, calls through names and
+    handles that were taken before, and a backward whose forward ran before.  In a process of its own."""
+    subprocess.run([sys.executable, "-c", f"HOW = {how!r}\n{_SECOND_LOAD}"], check=True, cwd=ROOT, timeout=300)
+
+
+def test_another_schema_of_a_registered_operator_is_refused():
+    from ads_model_kernel_library_b200.gdpa import ops
+
+    with pytest.raises(RuntimeError, match="another schema"):
+        ops._define_op("generalized_dot_product_attention(Tensor query) -> Tensor", None, None)
+    q, k, v, off = _meta()
+    assert _call(q, k, v, off, "relu").shape == q.shape
