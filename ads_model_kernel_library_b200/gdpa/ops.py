@@ -257,7 +257,9 @@ def _fill_fwd_params(q, k, v, o, qo, ko, batch, H, D, max_q, max_kv, scale, act_
     return p
 
 
-_below_autograd = getattr(torch._C, "_AutoDispatchBelowAutograd", None)  # private, as above: without it, the public form
+# private, as above: without them, the public form
+_below_autograd = getattr(torch._C, "_AutoDispatchBelowAutograd", None)
+_keys_below_autograd = getattr(torch._C, "_after_autograd_keyset", None)
 _untraced = getattr(torch, "_disable_dynamo", torch.compiler.disable)  # the first imports the compiler when it is used, not now
 
 # The operators belong to the process, not to this module: torch keeps the handle of an operator that it has once looked up
@@ -277,16 +279,16 @@ class _Gradient(torch.autograd.Function):
     """A call that needs a gradient: the operator below autograd, and its ``backward``."""
 
     @staticmethod
-    def forward(ctx, functions, overload, *args):
+    def forward(ctx, functions, below, keys, *args):
         ctx.functions = functions  # this call's own, should the operator get others before its backward
         with _below_autograd():
-            output = overload(*args)
+            output = below(keys, *args)
         functions.setup_context(ctx, args, output)
         return output
 
     @staticmethod
     def backward(ctx, *grads):
-        return (None, None, *ctx.functions.backward(ctx, *grads))
+        return (None, None, None, *ctx.functions.backward(ctx, *grads))
 
 
 class _Operator:
@@ -301,23 +303,26 @@ class _Operator:
         overload = getattr(torch.ops.gdpa, name).default
         defaults = tuple(a.default_value for a in overload._schema.arguments)
 
-        def autograd_kernel(*args):
+        below = overload.redispatch  # on to the next kernel of this call: a second call would be another one in a profile
+
+        def autograd_kernel(keys, *args):
+            keys = keys & _keys_below_autograd
             if torch.is_grad_enabled():
                 for a in args:
                     if isinstance(a, torch.Tensor) and a.requires_grad:
-                        return _Gradient.apply(self.functions, overload, *args, *defaults[len(args):])
+                        return _Gradient.apply(self.functions, below, keys, *args, *defaults[len(args):])
             with _below_autograd():
-                return overload(*args)
+                return below(keys, *args)
 
         # the CUDA kernel is not traced into when it runs beneath a compiled caller
         self.library.impl(name, _untraced(lambda *args: self.functions.impl(*args)), "CUDA")
         torch.library.register_fake(f"gdpa::{name}", lambda *args: self.functions.fake(*args), lib=self.library)
-        if _below_autograd is None:
+        if _below_autograd is None or _keys_below_autograd is None:
             torch.library.register_autograd(f"gdpa::{name}", lambda ctx, *grads: self.functions.backward(ctx, *grads),
                                             setup_context=lambda *args, **kwargs: self.functions.setup_context(*args, **kwargs),
                                             lib=self.library)
         else:
-            self.library.impl(name, autograd_kernel, "Autograd")
+            self.library.impl(name, autograd_kernel, "Autograd", with_keyset=True)
 
 
 def _define_op(schema: str, impl, fake, setup_context=None, backward=None) -> None:

@@ -198,3 +198,37 @@ def test_another_schema_of_a_registered_operator_is_refused():
         ops._define_op("generalized_dot_product_attention(Tensor query) -> Tensor", None, None)
     q, k, v, off = _meta()
     assert _call(q, k, v, off, "relu").shape == q.shape
+
+
+@pytest.mark.parametrize("activation", ["relu", "softmax"])
+def test_a_profile_counts_a_call_once(activation):
+    """With a gradient and without one, the call and its backward are one event each."""
+    q, k, v, off = _meta()
+    name = "gdpa::generalized_dot_product_attention"
+    forward = name + ("_softmax" if activation == "softmax" else "")
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as trained:
+        out = _call(q, k, v, off, activation)
+        torch.autograd.grad(out, (q, k, v), torch.empty_like(out), create_graph=True)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as inferred, torch.no_grad():
+        _call(q, k, v, off, activation)
+    counts = [{e.key: e.count for e in p.key_averages() if e.key.startswith(name)} for p in (trained, inferred)]
+    assert counts == [{forward: 1, name + "_backward": 1}, {forward: 1}]
+
+
+def test_gradients_without_the_private_key_set():
+    """As without the dispatch guard: a torch without the set of keys that the gradient kernels pass on takes the public form."""
+    code = """
+import torch
+keys = getattr(torch._C, "_after_autograd_keyset", None)
+if keys is not None:
+    del torch._C._after_autograd_keyset
+from ads_model_kernel_library_b200.gdpa import ops
+if keys is not None:
+    torch._C._after_autograd_keyset = keys  # torch's own registration uses it under this name
+assert ops._keys_below_autograd is None
+q = torch.empty(10, 2, 64, dtype=torch.bfloat16, device="meta", requires_grad=True)
+off = torch.empty(3, dtype=torch.int64, device="meta")
+out = ops.generalized_dot_product_attention(q, q, q, off, off, 5, 5, activation="relu")
+assert torch.autograd.grad(out, q, torch.empty_like(out))[0].shape == q.shape
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT, timeout=300)
