@@ -338,7 +338,7 @@ def _define_op(schema: str, impl, fake, setup_context=None, backward=None) -> No
             pass
 
         def backward(ctx, *grads):
-            raise RuntimeError(f"Trying to backward through gdpa::{name} but it has no gradient")
+            raise RuntimeError(f"gdpa::{name} has no gradient: its outputs cannot be differentiated")
 
     functions = _Functions(impl, fake, setup_context, backward)
     operator = _operators.get(name)
