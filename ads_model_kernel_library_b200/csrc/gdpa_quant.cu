@@ -370,8 +370,10 @@ __global__ void __launch_bounds__(kTile) gdpa_quant_fp8_kernel(const QuantArgs a
 // rows.  x / scale: with the correctly rounded r = 1 / scale, q = x r and the exact remainder x - q scale,
 // q + remainder r is the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990), two fused operations a value
 // in place of a division; the exponents cannot leave the normal range where the result is not zero, because
-// scale >= 1e-12 and |x| <= 448 scale (1 + 2^-23).  A block that holds an infinity has an infinite scale and divides, and so
-// does one that holds a NaN.
+// scale >= 1e-12 and |x| <= 448 scale (1 + 2^-23).  It starts from -x: q = (-x) (-r), remainder q scale + (-x), quotient
+// q + remainder (-r), which for x = -0 is -0 + (+0) (-r) = -0, as a division gives it; from x and r it would be -0 + +0 = +0.
+// The sign is turned where the bf16 pair is widened, at no cost.  A block that holds an infinity has an infinite scale and
+// divides, and so does one that holds a NaN.
 // What keeps it from the copy rate is that a CTA waits for the offsets, reads, finds the maximum, converts and writes one
 // after the other, so it needs as many CTAs as fit and little arithmetic between their phases: maxima as integers (a NaN
 // shows in them, and the values of a block without one need no test), packed products.  1 143 311 tokens of 4 heads of 128
@@ -437,7 +439,7 @@ __global__ void __launch_bounds__(kQuantThreads, 4) gdpa_quant_fp8_tile_kernel(c
   if (t == 0) a.scales[g * a.heads + h] = scale;
   const float inv = 1.f / scale;
   const bool plain = !has_nan && amax_bits < 0x7f80u;
-  const uint64_t inv2 = pack_f32x2(inv, inv), neg_scale2 = pack_f32x2(-scale, -scale);
+  const uint64_t neg_inv2 = pack_f32x2(-inv, -inv), scale2 = pack_f32x2(scale, scale);
 #pragma unroll
   for (int i = 0; i < kPieces; ++i) {
     const int row = row_first + i * kRowStep;
@@ -446,13 +448,15 @@ __global__ void __launch_bounds__(kQuantThreads, 4) gdpa_quant_fp8_tile_kernel(c
     float v[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xffff0000u);
+      const uint64_t neg_x2 = pack_f32x2(__uint_as_float(w[j] * 0x10000u + 0x80000000u),
+                                         __uint_as_float((w[j] & 0xffff0000u) ^ 0x80000000u));
       if (plain) {
-        const uint64_t x2 = pack_f32x2(lo, hi), q = mul_f32x2(x2, inv2);
-        unpack_f32x2(fma_f32x2(fma_f32x2(q, neg_scale2, x2), inv2, q), v[2 * j], v[2 * j + 1]);
+        const uint64_t q = mul_f32x2(neg_x2, neg_inv2);
+        unpack_f32x2(fma_f32x2(fma_f32x2(q, scale2, neg_x2), neg_inv2, q), v[2 * j], v[2 * j + 1]);
       } else {
-        v[2 * j] = fmaxf(lo / scale, -448.f);  // also what a NaN becomes
-        v[2 * j + 1] = fmaxf(hi / scale, -448.f);
+        unpack_f32x2(neg_x2, v[2 * j], v[2 * j + 1]);
+        v[2 * j] = fmaxf(-v[2 * j] / scale, -448.f);  // also what a NaN becomes
+        v[2 * j + 1] = fmaxf(-v[2 * j + 1] / scale, -448.f);
       }
     }
     // the conversion saturates at +-448

@@ -29,3 +29,27 @@ def test_blocks_with_nan_and_infinity(head_dim):
     want = torch.where(x.isfinite(), r8.view(torch.uint8), torch.tensor(0xFE, dtype=torch.uint8))  # 0xFE: -448
     assert torch.equal(blocks.cpu(), rblocks) and torch.equal(scales.cpu()[:6], rscales)
     assert torch.equal(x8.cpu().view(torch.uint8), want)
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("lengths", [[300, 129], [1, 40]])
+@pytest.mark.parametrize("head_dim", [32, 64, 128])
+def test_a_negative_zero_keeps_its_sign(head_dim, lengths, fp32):
+    """Of both kernels, in blocks of finite values, blocks with an infinity and blocks of zeros only: -0, and what is so small
+    that it is rounded to it."""
+    import ads_model_kernel_library_b200.gdpa as G
+
+    off = torch.tensor([0, *torch.tensor(lengths).cumsum(0)])
+    x = torch.randn(int(off[-1]), 3, head_dim, generator=torch.Generator().manual_seed(7))
+    x = x.to(torch.float32 if fp32 else torch.bfloat16)
+    x[:, 0, ::3] = -0.0
+    x[:, 0, 1::5] = 0.0
+    x[:, 1] = -0.0
+    x[:, 1, ::2] = 0.0
+    x[:, 0, 2::7] = -1e-30
+    x[-1, 2, :5] = torch.tensor([-float("inf"), -0.0, 0.0, -1.0, 1.0])
+    x8, scales, _ = G.quantize_fp8_blockwise(x.cuda(), off.cuda())
+    r8, rscales, _ = orc.quantize_fp8_blockwise(x.nan_to_num(0, float("inf"), -float("inf")), off)
+    want = torch.where(x.isfinite(), r8.view(torch.uint8), torch.tensor(0xFE, dtype=torch.uint8))
+    assert torch.equal(scales.cpu()[: rscales.shape[0]], rscales)
+    assert torch.equal(x8.cpu().view(torch.uint8), want)
