@@ -279,16 +279,17 @@ class _Gradient(torch.autograd.Function):
     """A call that needs a gradient: the operator below autograd, and its ``backward``."""
 
     @staticmethod
-    def forward(ctx, functions, below, keys, *args):
+    def forward(ctx, call, *args):
+        functions, redispatch, keys = call
         ctx.functions = functions  # this call's own, should the operator get others before its backward
         with _below_autograd():
-            output = below(keys, *args)
+            output = redispatch(keys, *args)
         functions.setup_context(ctx, args, output)
         return output
 
     @staticmethod
     def backward(ctx, *grads):
-        return (None, None, None, *ctx.functions.backward(ctx, *grads))
+        return (None, *ctx.functions.backward(ctx, *grads))
 
 
 class _Operator:
@@ -303,16 +304,16 @@ class _Operator:
         overload = getattr(torch.ops.gdpa, name).default
         defaults = tuple(a.default_value for a in overload._schema.arguments)
 
-        below = overload.redispatch  # on to the next kernel of this call: a second call would be another one in a profile
+        redispatch = overload.redispatch
 
         def autograd_kernel(keys, *args):
-            keys = keys & _keys_below_autograd
             if torch.is_grad_enabled():
                 for a in args:
                     if isinstance(a, torch.Tensor) and a.requires_grad:
-                        return _Gradient.apply(self.functions, below, keys, *args, *defaults[len(args):])
+                        # on to the next kernel of this call: within a node of its own, a second call would be another one in a profile
+                        return _Gradient.apply((self.functions, redispatch, keys & _keys_below_autograd), *args, *defaults[len(args):])
             with _below_autograd():
-                return below(keys, *args)
+                return overload(*args)
 
         # the CUDA kernel is not traced into when it runs beneath a compiled caller
         self.library.impl(name, _untraced(lambda *args: self.functions.impl(*args)), "CUDA")
