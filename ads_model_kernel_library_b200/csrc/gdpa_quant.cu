@@ -492,12 +492,16 @@ int launch_quant_fp8(const QuantArgs& a, int in_is_fp32, cudaStream_t stream) {
   if (cudaGetLastError() != cudaSuccess) return GDPA_ERR_LAUNCH_;
   if (a.max_blocks == 0) return 0;
   // The two head dims the forward takes; the other sizes, fp32 and unaligned tensors go through the general kernel, and so
-  // would more tiles than a 1-D grid holds, and batches whose sequences have fewer than 80 rows on average: with a few rows
-  // a tile the time is that of a CTA's dependent loads, and three times as many of the general kernel's CTAs are resident
-  // (524 288 rows of 4 heads of 128 in sequences of 8 rows 1630 us here and 1001 us there, of 64 rows 295 and 280, of 96 rows
-  // 260 and 263, of 2000 rows 190 and 229).
+  // would more tiles than a 1-D grid holds, and batches whose sequences have fewer than 8192 values a head on average (64 rows
+  // of 128, 128 rows of 64): with little in a tile the time is that of a CTA's dependent loads, and twelve of the general
+  // kernel's CTAs are resident where four of this one are.  Whole calls, 2^28 values of 4 heads, every sequence of
+  // that length / lengths from 1 to twice that, us here and there:
+  //   of 128:   8 rows 1687 / 1659 and  977 / 992;   56 rows 282 / 283 and 268 / 279;   64 rows 265 / 269 and 261 / 275;
+  //            80 rows  221 / 244  and  248 / 264; 2000 rows 156 / 158 and 225 / 226
+  //   of 64:   64 rows  423 / 412  and  356 / 375;   96 rows 281 / 333 and 287 / 316;  128 rows 246 / 308 and 268 / 299;
+  //           160 rows  293 / 279  and  280 / 283; 2000 rows 198 / 200 and 237 / 237
   if (!in_is_fp32 && a.vec16 && (a.head_dim == 64 || a.head_dim == 128) && a.max_blocks * a.heads < (1ll << 31) &&
-      a.total >= 80ll * a.batch) {
+      static_cast<long long>(a.total) * a.head_dim >= 8192ll * a.batch) {
     const unsigned tiles = static_cast<unsigned>(a.max_blocks * a.heads);
     if (a.head_dim == 64) gdpa_quant_fp8_tile_kernel<64><<<tiles, kQuantThreads, 0, stream>>>(a);
     else gdpa_quant_fp8_tile_kernel<128><<<tiles, kQuantThreads, 0, stream>>>(a);

@@ -53,3 +53,21 @@ def test_a_negative_zero_keeps_its_sign(head_dim, lengths, fp32):
     want = torch.where(x.isfinite(), r8.view(torch.uint8), torch.tensor(0xFE, dtype=torch.uint8))
     assert torch.equal(scales.cpu()[: rscales.shape[0]], rscales)
     assert torch.equal(x8.cpu().view(torch.uint8), want)
+
+
+@pytest.mark.parametrize("offset_dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("rows", [-1, 0, 1])
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_both_sides_of_the_rule_by_average_length(head_dim, rows, offset_dtype):
+    """One row less than the one-pass kernel takes (8192 values a sequence and head on average), as many, and one more."""
+    import ads_model_kernel_library_b200.gdpa as G
+
+    lens = [1, 0, 127, 128, 129, 40, 3, 128, 20]
+    lens += [8192 // head_dim * (len(lens) + 1) + rows - sum(lens)]
+    assert lens[-1] > 0
+    off = torch.tensor([0, *torch.tensor(lens).cumsum(0)], dtype=offset_dtype)
+    x = torch.randn(sum(lens), 3, head_dim, generator=torch.Generator().manual_seed(head_dim)).to(torch.bfloat16)
+    x8, scales, blocks = G.quantize_fp8_blockwise(x.cuda(), off.cuda())
+    r8, rscales, rblocks = orc.quantize_fp8_blockwise(x, off)
+    assert torch.equal(blocks.cpu(), rblocks) and torch.equal(scales.cpu()[: rscales.shape[0]], rscales)
+    assert torch.equal(x8.cpu().view(torch.uint8), r8.view(torch.uint8))
