@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kTile) gdpa_quant_fp8_kernel(const QuantArgs a
 // after the other, so it needs as many CTAs as fit and little arithmetic between their phases: maxima as integers (a NaN
 // shows in them, and the values of a block without one need no test), packed products.  1 143 311 tokens of 4 heads of 128
 // (264 us at the copy rate): 394 us with a maximum and a clamp in floating point, 375 us without them in 80 registers (three
-// CTAs an SM), 327 us in 64 (four), 340 us in 48 (five, with spills); reading the tile twice in 16-value pieces 472 us;
+// CTAs an SM), 330 us in 64 (four), 340 us in 48 (five, with spills); reading the tile twice in 16-value pieces 472 us;
 // a CTA that takes four heads one after another, each read under the one before, 388 us.
 constexpr int kQuantThreads = 256;
 template <int D>

@@ -246,8 +246,9 @@ __host__ __device__ constexpr uint32_t umma_idesc(uint32_t a_fmt, uint32_t b_fmt
 
 // D[tmem] (+)= A[smem] * B[smem].  Called by a whole warp, whose elected thread (always the same) issues for the CTA: the
 // instruction takes its operands from uniform registers, and in code that the warp runs together with values that are the
-// same for its lanes (warp_uniform) the compiler keeps them there; under a branch on the lane it moves each of them over
-// for each instruction.
+// same for its lanes (warp_uniform) they stay there; code under a branch on the lane fills them anew for each instruction
+// (warp instructions for the same products, forward and backward of 48 sequences of 512 to 4096 tokens: 467.6 -> 454.2 M and
+// 1164 -> 1103 M; tensor pipe 61 -> 68 % and 60 -> 65 % active).
 __device__ __forceinline__ void umma_ss_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                             uint32_t accumulate) {
   asm volatile(
