@@ -331,8 +331,8 @@ def _define_op(schema: str, impl, fake, setup_context=None, backward=None) -> No
     that is there already (this module is run a second time) gets them in place of its own.  Without ``backward``
     differentiating the outputs raises.
 
-    A call on a few short sequences is host time only, a fifth of it the generic form's with a gradient and a seventh
-    without: forward and backward of eight sequences 278 -> 220 us, the forward of four requests with shared KV 60 -> 51 us."""
+    A call on a few short sequences is host time only, a sixth of it the generic form's with a gradient and a twelfth
+    without: forward and backward of eight sequences 278 -> 229 us, the forward of four requests with shared KV 59.8 -> 54.9 us."""
     name = schema[:schema.index("(")]
     if backward is None:
         def setup_context(ctx, inputs, output):
